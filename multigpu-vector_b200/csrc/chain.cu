@@ -88,44 +88,74 @@ __device__ uint32_t sink_chunk(const SinkView& s, uint32_t c, bool opener, uint3
     }
 }
 
-// Append `my_cnt` rows per lane, reserved warp-wide; row_val(i, col).
-template <class RowFn>
-__device__ __forceinline__ void sink_emit_warp(const SinkView& s, uint32_t my_cnt, RowFn row_val, uint32_t* err) {
+// A warp's output rows on their way to the sink: the probe row's offset and
+// the match's build payload.  The rows' columns are read when the staging is
+// flushed, kSinkStage rows at a time under one reservation: a sink has one
+// row cursor, and same-address atomics retire one after another in L2 (a
+// reservation per 32 matches held the 8 M-row join -> sink at 931 us).
+constexpr uint32_t kSinkStage = 512;
+struct SinkStage {
+    uint32_t row[kSinkStage];
+    int32_t pay[kSinkStage];
+};
+
+// Writes the `n` staged rows of a warp (n <= kSinkStage) to the sink: output
+// column c is input column a.ref[c] of the staged row, or its build payload.
+// Consecutive lanes write consecutive rows, one column after another.
+__device__ __noinline__ void sink_flush(const ChainDev& a, const SinkStage& st, uint32_t n, uint32_t* err) {
+    const SinkView& s = a.sink;
     const uint32_t lane = lane_id();
-    uint32_t incl = my_cnt;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= (uint32_t)o) incl += y;
-    }
-    const uint32_t total = __shfl_sync(0xffffffffu, incl, 31);
-    if (total == 0) return;
+    __syncwarp();
+    if (n == 0) return;
     unsigned long long base = 0;
-    if (lane == 0) base = atomicAdd(s.cursor, (unsigned long long)total);
+    if (lane == 0) base = atomicAdd(s.cursor, (unsigned long long)n);
     base = __shfl_sync(0xffffffffu, base, 0);
     const unsigned long long limit = (unsigned long long)s.max_chunks * s.capacity;
     const unsigned long long first_c = base / s.capacity;
-    const unsigned long long last_c = (base + total - 1) / s.capacity;
+    const unsigned long long last_c = (base + n - 1) / s.capacity;
+    const unsigned long long first_off = base - first_c * s.capacity;
+    // lane l looks after chunk first_c + l; the chunks this warp owns are opened before any is waited for
     uint32_t my_chunk_id = kNil - 1;
     const unsigned long long c = first_c + lane;
-    if (c <= last_c && c < s.max_chunks) {
-        const bool opener = c * s.capacity >= base;  // this warp owns the chunk's first row
-        my_chunk_id = sink_chunk(s, (uint32_t)c, opener, err);
-    }
+    const bool mine = c <= last_c && c < s.max_chunks;
+    const bool opener = mine && c * s.capacity >= base;
+    if (opener) my_chunk_id = sink_chunk(s, (uint32_t)c, true, err);
     __syncwarp();
-    if (lane == 0 && (last_c - first_c >= 32 || base + total > limit)) set_error(err, kDevOverflow, 5);
-    const uint32_t maxc = __reduce_max_sync(0xffffffffu, my_cnt);
-    const unsigned long long pos0 = base + incl - my_cnt;
-    for (uint32_t i = 0; i < maxc; ++i) {
-        const bool act = i < my_cnt;
-        const unsigned long long pos = pos0 + i;
-        const unsigned long long rel = act ? pos / s.capacity - first_c : 0ull;
-        const uint32_t id = __shfl_sync(0xffffffffu, my_chunk_id, (int)(rel & 31ull));
-        if (!act || pos >= limit || rel >= 32 || id >= s.pool->nbuffers) continue;
-        const uint32_t off = (uint32_t)(pos % s.capacity);
-        int32_t* base_ptr = s.slab + (size_t)id * s.pool_ncols * s.capacity;
-        for (uint32_t col = 0; col < s.ncols; ++col) base_ptr[(size_t)col * s.capacity + off] = row_val(i, col);
+    if (mine && !opener) my_chunk_id = sink_chunk(s, (uint32_t)c, false, err);
+    __syncwarp();
+    if (lane == 0 && (last_c - first_c >= 32 || base + n > limit)) set_error(err, kDevOverflow, 5);
+    for (uint32_t i0 = 0; i0 < n; i0 += 4 * 32) {
+        // where the lane's four rows of this step go, and what they are
+        int32_t* dst[4];
+        uint32_t row[4];
+        int32_t pay[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const uint32_t i = i0 + u * 32 + lane;
+            unsigned long long off = first_off + i;
+            uint32_t rel = 0;
+            while (off >= s.capacity && rel < 32) {
+                off -= s.capacity;
+                ++rel;
+            }
+            const uint32_t id = __shfl_sync(0xffffffffu, my_chunk_id, (int)(rel & 31u));
+            const bool ok = i < n && base + i < limit && rel < 32 && id < s.pool->nbuffers;
+            dst[u] = ok ? s.slab + (size_t)id * s.pool_ncols * s.capacity + off : nullptr;
+            row[u] = ok ? st.row[i] : 0u;
+            pay[u] = ok ? st.pay[i] : 0;
+        }
+        for (uint32_t col = 0; col < s.ncols; ++col) {
+            const int32_t ref = a.ref[col];
+            int32_t v[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+                v[u] = ref == kBP ? pay[u] : (dst[u] ? __ldg(a.cols[ref] + row[u]) : 0);
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+                if (dst[u]) dst[u][(size_t)col * s.capacity] = v[u];
+        }
     }
+    __syncwarp();  // the staging is free again
 }
 
 // ---- group tables ------------------------------------------------------------
@@ -422,8 +452,9 @@ __device__ __forceinline__ void chain_windows(const ChainDev& a, bool unique, ui
                                               uint64_t win_first, uint64_t win_stride, uint32_t* ids,
                                               const SmemGroups& sg, unsigned long long& acnt,
                                               unsigned long long& asum, uint32_t* err,
-                                              const CellCtx* cc = nullptr) {
-    constexpr int NS = TERM == kTermSink ? MGV_MAX_COLS : kMaxTermSlots;
+                                              const CellCtx* cc = nullptr, SinkStage* stage = nullptr) {
+    // carried columns: a sink reads its columns when it flushes, so only the probe key is carried
+    constexpr int NS = TERM == kTermSink ? 1 : kMaxTermSlots;
     // A batch query's carried slots are fixed (FIXED): key, group, value from
     // input columns 0, 2, 3, so every slot pick below resolves at compile time.
     const uint32_t nslots = FIXED ? 3u : a.nslots;
@@ -434,10 +465,22 @@ __device__ __forceinline__ void chain_windows(const ChainDev& a, bool unique, ui
     const uint32_t lane = lane_id();
     const uint32_t len = (uint32_t)(row_hi - row_lo);
     const uint64_t stream_policy = l2_policy_evict_first();  // columns are read once; the join table stays
+    uint32_t staged = 0;  // sink: rows in the warp's staging
+    const uint32_t lt = (1u << lane) - 1u;
 
-    // push `cnt` (<= 128) offsets of the ring starting at `start`
+    // sink: room in the staging for one match per row of a vector
+    auto make_room = [&]() {
+        if (staged > kSinkStage - 128) {
+            sink_flush(a, *stage, staged, err);
+            staged = 0;
+        }
+    };
+
+    // push `cnt` (<= 128) rows: the ring's offsets from `start` on, or without
+    // a select the rows from `start` on themselves
     auto push_vector = [&](uint32_t start, uint32_t cnt) {
         __syncwarp();
+        if (TERM == kTermSink) make_room();
         uint32_t rid[4];
         uint32_t rng[4];  // shared scan: each row's filter range
         bool in[4];
@@ -445,7 +488,7 @@ __device__ __forceinline__ void chain_windows(const ChainDev& a, bool unique, ui
         for (int j = 0; j < 4; ++j) {
             const uint32_t idx = j * 32 + lane;
             in[j] = idx < cnt;
-            rid[j] = ids[(start + idx) & (kIdRing - 1)];
+            rid[j] = SEL ? ids[(start + idx) & (kIdRing - 1)] : start + idx;
             rng[j] = 0;
             if (TERM == kTermCells) {
                 rng[j] = rid[j] >> kCellRowBits;
@@ -458,7 +501,10 @@ __device__ __forceinline__ void chain_windows(const ChainDev& a, bool unique, ui
             const bool carried = (uint32_t)c < nslots;
             const int32_t* col = carried ? slot_col(c) + row_lo : nullptr;
 #pragma unroll
-            for (int j = 0; j < 4; ++j) v[c][j] = (carried && in[j]) ? ld_stream1(col + rid[j], stream_policy) : 0;
+            for (int j = 0; j < 4; ++j)  // a sink's flush reads the key again: no evict-first for it
+                v[c][j] = !(carried && in[j])  ? 0
+                          : TERM == kTermSink ? __ldg(col + rid[j])
+                                              : ld_stream1(col + rid[j], stream_policy);
         }
         // value of terminal reference r for the lane's row j and build payload bp
         auto val = [&](int32_t ref, int j, int32_t bp) -> int32_t {
@@ -483,8 +529,17 @@ __device__ __forceinline__ void chain_windows(const ChainDev& a, bool unique, ui
             } else if (TERM == kTermCells) {
                 if (active) cells_add_row(cc->sc, a.cells, rng[j], val(ref0, j, bp), val(ref1, j, bp), err);
             } else {
-                sink_emit_warp(
-                    a.sink, active ? 1u : 0u, [&](uint32_t, uint32_t col) { return val(a.ref[col], j, bp); }, err);
+                const unsigned m = __ballot_sync(0xffffffffu, active);
+                if (active) {
+                    const uint32_t pos = staged + __popc(m & lt);
+                    stage->row[pos] = rid[j];
+                    stage->pay[pos] = bp;
+                }
+                staged += __popc(m);
+                if (PROBE && !unique && staged > kSinkStage - 32) {  // a row may have any number of matches
+                    sink_flush(a, *stage, staged, err);
+                    staged = 0;
+                }
             }
         };
         if (!PROBE) {
@@ -507,8 +562,6 @@ __device__ __forceinline__ void chain_windows(const ChainDev& a, bool unique, ui
                 key[j] = pick_slot<NS>(v, probe_slot, j);
                 live[j] = in[j] && key[j] != kEmptyKey;
                 reserved_any |= in[j] && key[j] == kEmptyKey;
-                b[j] = home_bucket(key[j], a.table);
-                if (live[j]) ld_bucket(slots + 4ull * b[j], w[j]);
             }
             if (__any_sync(0xffffffffu, reserved_any)) {  // INT32_MIN keys join every side-list row
                 const uint32_t side_n =
@@ -517,15 +570,45 @@ __device__ __forceinline__ void chain_windows(const ChainDev& a, bool unique, ui
                 for (int j = 0; j < 4; ++j) {
                     const bool r = in[j] && key[j] == kEmptyKey;
                     if (__any_sync(0xffffffffu, r))
-                        for (uint32_t i = 0; i < side_n; ++i) emit(r, j, a.table.side_pay[i]);
+                        for (uint32_t i = 0; i < side_n; ++i) {
+                            emit(r, j, a.table.side_pay[i]);
+                            if (TERM == kTermSink) make_room();  // even a table of distinct keys may list many such rows
+                        }
                 }
+            }
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                b[j] = home_bucket(key[j], a.table);
+                if (live[j]) ld_bucket(slots + 4ull * b[j], w[j]);
             }
             const bool ko = a.table.key_only != 0;  // eight keys per bucket, payloads 0
             for (uint32_t round = 0; round <= nbuckets; ++round) {
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
                     const uint32_t k = (uint32_t)key[j];
-                    if (ko) {
+                    if (TERM == kTermSink) {
+                        // the bucket's matching slots as bits, emitted one per lane and
+                        // step: one emission site per row instead of one per slot, which
+                        // spilled 500 bytes
+                        uint32_t hits = 0;
+                        if (ko) {
+#pragma unroll
+                            for (int q = 0; q < 8; ++q) hits |= (uint32_t)(w[j][q] == k) << q;
+                        } else {
+#pragma unroll
+                            for (int q = 0; q < 4; ++q) hits |= (uint32_t)(w[j][2 * q] == k) << q;
+                        }
+                        if (!live[j]) hits = 0;
+                        const bool full = (ko ? w[j][7] : w[j][6]) != (uint32_t)kEmptyKey;
+                        live[j] = live[j] && full && !(unique && hits);
+                        while (__any_sync(0xffffffffu, hits != 0)) {
+                            const uint32_t q = __ffs(hits);  // 1-based
+                            const int32_t bp = ko ? 0
+                                                  : (int32_t)(q == 1 ? w[j][1] : q == 2 ? w[j][3] : q == 3 ? w[j][5] : w[j][7]);
+                            emit(hits != 0, j, bp);
+                            hits &= hits - 1;
+                        }
+                    } else if (ko) {
                         if (unique) {  // at most one match per run
                             bool f = false;
 #pragma unroll
@@ -573,56 +656,77 @@ __device__ __forceinline__ void chain_windows(const ChainDev& a, bool unique, ui
     };
 
     const int32_t* __restrict__ fcol = SEL ? a.cols[a.sel_col] + row_lo : nullptr;
-    const uint32_t lt = (1u << lane) - 1u;
     const uint64_t nwin = (len + kWinRows - 1) / kWinRows;
     uint32_t head = 0, fill = 0;  // fill < 128 between windows
     for (uint64_t win = win_first; win < nwin; win += win_stride) {
         const uint32_t r0 = (uint32_t)win * kWinRows;
-        int32_t f[kWinRows / 32];
+        if (!SEL) {  // every row qualifies: no ring
+            const uint32_t r1 = min(len - r0, (uint32_t)kWinRows) + r0;
+#pragma unroll 1
+            for (uint32_t r = r0; r < r1; r += 128) push_vector(r, min(r1 - r, 128u));
+        }
         if (SEL) {
+            int32_t f[kWinRows / 32];
 #pragma unroll
             for (int k = 0; k < kWinRows / 32; ++k) {
                 const uint32_t row = r0 + k * 32 + lane;
                 f[k] = row < len ? ld_stream1(fcol + row, stream_policy) : 0;
             }
-        }
 #pragma unroll
-        for (int k = 0; k < kWinRows / 32; ++k) {
-            const uint32_t row = r0 + k * 32 + lane;
-            const bool pass = row < len && (!SEL || f[k] <= a.sel_bound);
-            const unsigned m = __ballot_sync(0xffffffffu, pass);
-            if (pass) {
-                uint32_t e = row;
-                if (TERM == kTermCells) e |= cell_range_of(*cc, a.cells.m, f[k]) << kCellRowBits;
-                ids[(head + fill + __popc(m & lt)) & (kIdRing - 1)] = e;
+            for (int k = 0; k < kWinRows / 32; ++k) {
+                const uint32_t row = r0 + k * 32 + lane;
+                const bool pass = row < len && f[k] <= a.sel_bound;
+                const unsigned m = __ballot_sync(0xffffffffu, pass);
+                if (pass) {
+                    uint32_t e = row;
+                    if (TERM == kTermCells) e |= cell_range_of(*cc, a.cells.m, f[k]) << kCellRowBits;
+                    ids[(head + fill + __popc(m & lt)) & (kIdRing - 1)] = e;
+                }
+                fill += __popc(m);
             }
-            fill += __popc(m);
-        }
-        while (fill >= 128) {
-            push_vector(head, 128);
-            head = (head + 128) & (kIdRing - 1);
-            fill -= 128;
+            while (fill >= 128) {
+                push_vector(head, 128);
+                head = (head + 128) & (kIdRing - 1);
+                fill -= 128;
+            }
         }
     }
     if (fill) push_vector(head, fill);
+    if (TERM == kTermSink) sink_flush(a, *stage, staged, err);
 }
 
-template <bool SEL, bool PROBE, int TERM>
-__global__ void __launch_bounds__(kChainBlock, 1) k_chain(ChainDev a, uint32_t* err) {
+// Shared layout of k_chain: [id rings (a select's) | group table or sink staging].
+// A sink chain keeps no group table and reads its output columns in the
+// flush, so its warps need fewer registers: two CTAs of 12 warps per SM hide
+// more of the bucket reads' latency than one of 16.
+constexpr int kSinkBlock = 384;
+template <int TERM>
+constexpr int chain_block() { return TERM == kTermSink ? kSinkBlock : kChainBlock; }
+template <bool SEL, int TERM>
+constexpr size_t chain_ring_bytes() {
+    return SEL ? (size_t)(chain_block<TERM>() / 32) * kIdRing * sizeof(uint32_t) : 0;
+}
+
+// UNIQUE: the table is known to have no duplicate keys (a sink's probe has no
+// flush, a call, inside its rounds then).
+template <bool SEL, bool PROBE, int TERM, bool UNIQUE = false>
+__global__ void __launch_bounds__(chain_block<TERM>(), TERM == kTermSink ? 2 : 1)
+    k_chain(const __grid_constant__ ChainDev a, uint32_t* err) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const uint32_t warp = threadIdx.x / 32;
-    // shared layout: [id rings | group table]
     uint32_t* rings = reinterpret_cast<uint32_t*>(smem_raw);
     SmemGroups sg{nullptr, nullptr, nullptr, nullptr, nullptr, 0};
     if (TERM == kTermGroupby && a.smem_groups) {
-        sg = smem_groups_at(smem_raw + kRingBytes, a.smem_groups);
+        sg = smem_groups_at(smem_raw + chain_ring_bytes<SEL, TERM>(), a.smem_groups);
         smem_groups_init(sg);
         __syncthreads();
     }
+    SinkStage* stage = TERM == kTermSink ? reinterpret_cast<SinkStage*>(smem_raw + chain_ring_bytes<SEL, TERM>()) + warp : nullptr;
     unsigned long long acnt = 0, asum = 0;
-    chain_windows<SEL, PROBE, TERM>(a, a.unique != 0, 0, a.n, (uint64_t)blockIdx.x * kChainWarps + warp,
-                                    (uint64_t)gridDim.x * kChainWarps, rings + (size_t)warp * kIdRing, sg,
-                                    acnt, asum, err);
+    constexpr uint64_t kWarps = chain_block<TERM>() / 32;
+    chain_windows<SEL, PROBE, TERM>(a, UNIQUE || a.unique != 0, 0, a.n, (uint64_t)blockIdx.x * kWarps + warp,
+                                    (uint64_t)gridDim.x * kWarps, rings + (size_t)warp * kIdRing, sg,
+                                    acnt, asum, err, nullptr, stage);
     if (TERM == kTermAgg) block_accumulate2<kChainBlock>(acnt, asum, a.acc);
     if (TERM == kTermGroupby && a.smem_groups) {
         __syncthreads();
@@ -887,13 +991,17 @@ cudaError_t launch_batch(const ChainDev* d_qs, const BatchOut* d_outs, const Bat
 }
 
 template <bool SEL, bool PROBE, int TERM>
-static cudaError_t launch_chain_t(const ChainDev& d, size_t smem, uint64_t n, cudaStream_t s, Context* ctx) {
-    auto k = k_chain<SEL, PROBE, TERM>;
+static cudaError_t launch_chain_t(const ChainDev& d, uint64_t n, cudaStream_t s, Context* ctx) {
+    auto k = PROBE && TERM == kTermSink && d.unique ? k_chain<SEL, PROBE, TERM, PROBE && TERM == kTermSink>
+                                                    : k_chain<SEL, PROBE, TERM>;
+    const size_t smem = chain_ring_bytes<SEL, TERM>() + smem_groups_bytes(d.smem_groups) +
+                        (TERM == kTermSink ? (kSinkBlock / 32) * sizeof(SinkStage) : 0);
+    constexpr int block = chain_block<TERM>();
     if (smem > 48 * 1024) {
         cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return e;
     }
-    const int full = occupancy_grid((const void*)k, kChainBlock, smem, ctx);
+    const int full = occupancy_grid((const void*)k, block, smem, ctx);
     // row offsets inside the kernel are 32-bit: launch at most 2^31 rows at a time
     constexpr uint64_t kChunk = 1ull << 31;
     for (uint64_t base = 0; base < n; base += kChunk) {
@@ -902,9 +1010,9 @@ static cudaError_t launch_chain_t(const ChainDev& d, size_t smem, uint64_t n, cu
         for (uint32_t i = 0; i < c.ncols; ++i)
             if (c.cols[i]) c.cols[i] += base;
         int grid = full;
-        const uint64_t need = ((c.n + kWinRows - 1) / kWinRows + kChainWarps - 1) / kChainWarps;
+        const uint64_t need = ((c.n + kWinRows - 1) / kWinRows + block / 32 - 1) / (block / 32);
         if ((uint64_t)grid > need) grid = (int)(need ? need : 1);
-        k<<<grid, kChainBlock, smem, s>>>(c, ctx->d_err);
+        k<<<grid, block, smem, s>>>(c, ctx->d_err);
         ctx->launches++;
         cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) return e;
@@ -913,12 +1021,12 @@ static cudaError_t launch_chain_t(const ChainDev& d, size_t smem, uint64_t n, cu
 }
 
 template <int TERM>
-static cudaError_t launch_chain_term(const ChainArgs& a, const ChainDev& d, size_t smem, cudaStream_t s, Context* ctx) {
+static cudaError_t launch_chain_term(const ChainArgs& a, const ChainDev& d, cudaStream_t s, Context* ctx) {
     if (!a.has_probe)
-        return a.has_sel ? launch_chain_t<true, false, TERM>(d, smem, a.n, s, ctx)
-                         : launch_chain_t<false, false, TERM>(d, smem, a.n, s, ctx);
-    return a.has_sel ? launch_chain_t<true, true, TERM>(d, smem, a.n, s, ctx)
-                     : launch_chain_t<false, true, TERM>(d, smem, a.n, s, ctx);
+        return a.has_sel ? launch_chain_t<true, false, TERM>(d, a.n, s, ctx)
+                         : launch_chain_t<false, false, TERM>(d, a.n, s, ctx);
+    return a.has_sel ? launch_chain_t<true, true, TERM>(d, a.n, s, ctx)
+                     : launch_chain_t<false, true, TERM>(d, a.n, s, ctx);
 }
 
 cudaError_t launch_chain(const ChainArgs& a, cudaStream_t s, Context* ctx) {
@@ -934,7 +1042,8 @@ cudaError_t launch_chain(const ChainArgs& a, cudaStream_t s, Context* ctx) {
     d.acc = a.acc;
     d.gt = a.gt;
     d.sink = a.sink;
-    // carried columns: the probe key and every column the terminal reads
+    // carried columns: the probe key and every column the terminal reads (a
+    // sink reads its columns by row when it flushes: its references stay input columns)
     int32_t slot_of[MGV_MAX_COLS];
     for (int c = 0; c < MGV_MAX_COLS; ++c) slot_of[c] = -1;
     auto carry = [&](int32_t col) -> int32_t {
@@ -948,16 +1057,16 @@ cudaError_t launch_chain(const ChainArgs& a, cudaStream_t s, Context* ctx) {
     };
     d.probe_slot = a.has_probe ? carry((int32_t)a.probe_col) : -1;
     d.nref = a.nref;
-    for (uint32_t i = 0; i < a.nref; ++i) d.ref[i] = carry(a.ref[i]);
+    for (uint32_t i = 0; i < a.nref; ++i)
+        d.ref[i] = a.term != kTermSink ? carry(a.ref[i]) : (uint32_t)a.ref[i] == a.ncols ? kBP : a.ref[i];
     if (a.term != kTermSink && d.nslots > (uint32_t)kMaxTermSlots) return cudaErrorInvalidValue;
     // the shared group table: as large as the global one (2 x max_groups, a
     // power of two), capped by the tuning's slot limit
     d.smem_groups = a.term == kTermGroupby ? std::min(a.smem_groups, a.gt.cap) : 0;
-    const size_t smem = kRingBytes + smem_groups_bytes(d.smem_groups);
     switch (a.term) {
-        case kTermAgg: return launch_chain_term<kTermAgg>(a, d, smem, s, ctx);
-        case kTermGroupby: return launch_chain_term<kTermGroupby>(a, d, smem, s, ctx);
-        default: return launch_chain_term<kTermSink>(a, d, smem, s, ctx);
+        case kTermAgg: return launch_chain_term<kTermAgg>(a, d, s, ctx);
+        case kTermGroupby: return launch_chain_term<kTermGroupby>(a, d, s, ctx);
+        default: return launch_chain_term<kTermSink>(a, d, s, ctx);
     }
 }
 

@@ -54,10 +54,13 @@ struct mgv_batch {
     BatchItem* d_probe_items = nullptr;
     BatchItem* d_compact_items = nullptr;
     uint32_t n_build = 0, n_probe = 0, n_compact = 0;
+    GroupSortJob* d_sorts = nullptr;  // queries whose groups are ordered on the device, largest first
+    uint32_t n_sorts = 0;
+    std::vector<uint8_t> ordered;  // per query: its landed rows are in group order
     std::vector<uint64_t> out_offset;  // first packed row of each query
-    // host landing zone: the packing kernel writes each query's rows straight into
-    // it (pinned, mapped), so only the groups found cross to the host, not every
-    // query's max_groups rows
+    // host landing zone: each query's rows are written straight into it (pinned,
+    // mapped), so only the groups found cross to the host, not every query's
+    // max_groups rows
     mgv_group_row* h_rows = nullptr;
     mgv_group_row* h_rows_dev = nullptr;  // the same memory as the device addresses it
     uint32_t* h_counts = nullptr;
@@ -72,6 +75,7 @@ struct mgv_batch {
     struct PlainQuery {
         mgv_op *hb = nullptr, *gb = nullptr, *probe = nullptr, *sel = nullptr;
         std::vector<mgv_group_row> rows;
+        bool sorted = false;  // by the group-by's close, else when read
     };
     std::vector<PlainQuery> plain;
 };
@@ -114,6 +118,7 @@ mgv_status enqueue_run(mgv_batch* b, cudaStream_t s) {
                                       b->total_regions, b->max_job_regions, b->rsc, true, false, s, ctx));
     MGV_CUDA_TRY(launch_batch(b->d_qs, b->d_outs, b->d_probe_items, b->n_probe, b->d_compact_items, b->n_compact,
                               (int)b->cfg.probe_ctas_per_sm, b->cfg.item_order, s, ctx));
+    MGV_CUDA_TRY(launch_group_sort(b->d_sorts, GroupSortJob{}, b->n_sorts, s, ctx));
     MGV_CUDA_TRY(cudaMemcpyAsync(b->h_counts, b->out_counts, sizeof(uint32_t) * b->q.size(), cudaMemcpyDeviceToHost, s));
     MGV_CUDA_TRY(cudaMemcpyAsync(b->h_err, ctx->d_err, 2 * sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
     return MGV_OK;
@@ -131,12 +136,12 @@ mgv_status check_run(mgv_batch* b) {
 
 void sort_rows(std::vector<mgv_group_row>& v) { sort_group_rows(v); }
 
-}  // namespace
+// Groups up to this many per query are ordered on the device when a batch has
+// the memory for it (40 bytes of packed rows and sorting space per group).
+constexpr uint32_t kDeviceOrderGroups = kDeviceOrderCap / 2;
 
-extern "C" {
-
-mgv_status mgv_batch_create(mgv_ctx* ctx, const mgv_query_desc* qs, uint32_t nq, const mgv_batch_config* config,
-                            mgv_batch** out) {
+mgv_status create_batch(mgv_ctx* ctx, const mgv_query_desc* qs, uint32_t nq, const mgv_batch_config* config,
+                        bool device_order, mgv_batch** out) {
     if (!ctx || (!qs && nq) || !out) return fail(MGV_EINVAL, "NULL argument");
     *out = nullptr;
     mgv_batch_config cfg{};
@@ -226,6 +231,19 @@ mgv_status mgv_batch_create(mgv_ctx* ctx, const mgv_query_desc* qs, uint32_t nq,
     }
     const size_t rsc_off = take(region_scratch_bytes(total_regions, build_total));
     const size_t outs_off = take(sizeof(BatchOut) * std::max(nq, 1u));
+    b->ordered.assign(nq, 0);
+    std::vector<uint32_t> sorts;
+    std::vector<size_t> rows_off(nq), pairs_off(nq);
+    for (uint32_t i = 0; device_order && i < nq; ++i) {
+        if (qs[i].max_groups > kDeviceOrderGroups) continue;
+        b->ordered[i] = 1;
+        sorts.push_back(i);
+        rows_off[i] = take(sizeof(mgv_group_row) * (size_t)qs[i].max_groups);
+        pairs_off[i] = take(2 * sizeof(unsigned long long) * (size_t)qs[i].max_groups);
+    }
+    std::stable_sort(sorts.begin(), sorts.end(),
+                     [&](uint32_t x, uint32_t y) { return qs[x].max_groups > qs[y].max_groups; });
+    const size_t sorts_off = take(sizeof(GroupSortJob) * std::max<size_t>(sorts.size(), 1));
     // work items
     std::vector<BatchItem> bi, pi, ci;
     for (uint32_t i = 0; i < nq; ++i) {
@@ -321,11 +339,23 @@ mgv_status mgv_batch_create(mgv_ctx* ctx, const mgv_query_desc* qs, uint32_t nq,
         c.smem_groups = std::min(gcap[i], kMaxSmemGroups);
         hj[i] = RegionJob{t, qs[i].build_keys, qs[i].build_payloads, nullptr, 0, region0[i],
                           (nbk[i] + kRegionBuckets - 1) / kRegionBuckets, 0};
-        ho[i] = BatchOut{g, b->h_rows_dev + b->out_offset[i], b->out_counts + i, qs[i].max_groups, 0};
+        // a query ordered on the device is packed there first
+        mgv_group_row* packed = b->ordered[i] ? reinterpret_cast<mgv_group_row*>(A + rows_off[i])
+                                              : b->h_rows_dev + b->out_offset[i];
+        ho[i] = BatchOut{g, packed, b->out_counts + i, qs[i].max_groups, 0};
     }
+    std::vector<GroupSortJob> hs;
+    for (uint32_t i : sorts)
+        hs.push_back(GroupSortJob{ho[i].rows, b->out_counts + i, reinterpret_cast<unsigned long long*>(A + pairs_off[i]),
+                                  b->h_rows_dev + b->out_offset[i], nullptr, nullptr, nullptr, qs[i].max_groups,
+                                  qs[i].max_groups});
+    b->d_sorts = reinterpret_cast<GroupSortJob*>(A + sorts_off);
+    b->n_sorts = (uint32_t)hs.size();
     e = cudaMemcpy(b->d_qs, hq.data(), sizeof(ChainDev) * nq, cudaMemcpyHostToDevice);
     if (e == cudaSuccess) e = cudaMemcpy(b->d_jobs, hj.data(), sizeof(RegionJob) * nq, cudaMemcpyHostToDevice);
     if (e == cudaSuccess) e = cudaMemcpy(b->d_outs, ho.data(), sizeof(BatchOut) * nq, cudaMemcpyHostToDevice);
+    if (e == cudaSuccess && !hs.empty())
+        e = cudaMemcpy(b->d_sorts, hs.data(), sizeof(GroupSortJob) * hs.size(), cudaMemcpyHostToDevice);
     if (e == cudaSuccess && !bi.empty())
         e = cudaMemcpy(b->d_build_items, bi.data(), sizeof(BatchItem) * bi.size(), cudaMemcpyHostToDevice);
     if (e == cudaSuccess && !pi.empty())
@@ -339,6 +369,20 @@ mgv_status mgv_batch_create(mgv_ctx* ctx, const mgv_query_desc* qs, uint32_t nq,
     }
     *out = b;
     return MGV_OK;
+}
+
+}  // namespace
+
+extern "C" {
+
+mgv_status mgv_batch_create(mgv_ctx* ctx, const mgv_query_desc* qs, uint32_t nq, const mgv_batch_config* config,
+                            mgv_batch** out) {
+    mgv_status st = create_batch(ctx, qs, nq, config, true, out);
+    if (st == MGV_ENOMEM) {
+        (void)cudaGetLastError();  // the failed allocation's
+        st = create_batch(ctx, qs, nq, config, false, out);
+    }
+    return st;
 }
 
 mgv_status mgv_batch_run(mgv_batch* b, void* stream) {
@@ -411,26 +455,39 @@ mgv_status mgv_batch_run_plain(mgv_batch* b, void* stream) {
     }
     b->last_ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
     // kept as closed (unordered); ordered when read, as the batch's own rows
-    for (uint32_t i = 0; i < nq; ++i) b->plain[i].rows = static_cast<Op*>(b->plain[i].gb)->gb_rows;
+    for (uint32_t i = 0; i < nq; ++i) {
+        const Op* g = static_cast<Op*>(b->plain[i].gb);
+        b->plain[i].rows.assign(g->gb_view, g->gb_view + g->gb_n);
+        b->plain[i].sorted = g->gb_sorted;
+    }
     return MGV_OK;
 }
 
 mgv_status mgv_batch_result(mgv_batch* b, uint32_t q, int plain, mgv_group_row* out, uint64_t cap, uint64_t* rows) {
     if (!b) return fail(MGV_EINVAL, "batch is NULL");
     if (q >= b->q.size()) return fail(MGV_EINVAL, "no such query");
-    std::vector<mgv_group_row> v;
+    const mgv_group_row* v = nullptr;
+    uint64_t n = 0;
+    std::vector<mgv_group_row> sorted;
     if (plain) {
         if (b->plain.empty()) return fail(MGV_ESTATE, "the plain pipeline has not run");
-        v = b->plain[q].rows;
-        sort_rows(v);
+        auto& p = b->plain[q];
+        if (!p.sorted) sort_rows(p.rows);
+        p.sorted = true;
+        v = p.rows.data();
+        n = p.rows.size();
     } else {
         if (!b->warmed) return fail(MGV_ESTATE, "the batch has not run");
-        const uint32_t n = std::min<uint32_t>(b->h_counts[q], b->q[q].max_groups);
-        v.assign(b->h_rows + b->out_offset[q], b->h_rows + b->out_offset[q] + n);
-        sort_rows(v);
+        v = b->h_rows + b->out_offset[q];
+        n = std::min<uint32_t>(b->h_counts[q], b->q[q].max_groups);
+        if (!b->ordered[q]) {
+            sorted.assign(v, v + n);
+            sort_rows(sorted);
+            v = sorted.data();
+        }
     }
-    if (rows) *rows = v.size();
-    if (out) std::memcpy(out, v.data(), sizeof(mgv_group_row) * std::min<uint64_t>(cap, v.size()));
+    if (rows) *rows = n;
+    if (out) std::memcpy(out, v, sizeof(mgv_group_row) * std::min<uint64_t>(cap, n));
     return MGV_OK;
 }
 

@@ -111,46 +111,57 @@ void sort_group_rows(std::vector<mgv_group_row>& v) {
 
 }  // namespace mgv
 
-// A terminal group-by's close: its groups are packed on the device and come
-// back with the error word in one copy to pinned memory and one
-// synchronisation.  They are ordered by group when first read.
-// Group rows read back together with the count at a group-by's close; a
-// larger result costs one more copy (most results are smaller).
-constexpr uint32_t kGroupRowsFirstCopy = 4096;
+// A terminal group-by's close: its groups come out of the table, in group
+// order, straight into the operator's pinned landing zone with the error word
+// and their count; one synchronisation.  The kernels leave the table empty, so
+// the next open has nothing to clear.  A table of up to kSmallGroupCap slots
+// takes one kernel of one CTA (a table that size is read in a few
+// microseconds); a larger one is packed by the whole GPU and ordered by one
+// CTA; one past kDeviceOrderCap slots (half a GiB of sorting space and up) is
+// ordered by the host when its result is read, and so is one of at most
+// kHostOrderGroups groups (a microsecond on the host).
+constexpr uint32_t kHostOrderGroups = 64;
 
 static mgv_status close_groupby(Op* o, cudaStream_t s) {
     Context* ctx = o->ctx;
-    unsigned char* h = o->gb_land;
-    MGV_CUDA_TRY(cudaMemsetAsync(o->gb_dev_count, 0, sizeof(uint32_t), s));
-    MGV_CUDA_TRY(launch_group_pack(o->gtab, o->gb_dev_rows, o->gb_dev_count, s, ctx));
-    MGV_CUDA_TRY(cudaMemcpyAsync(h, ctx->d_err, 2 * sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
-    MGV_CUDA_TRY(cudaMemcpyAsync(h + 8, o->gb_dev_count, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
-    // the first rows come with the count; a larger result follows after it
-    const uint32_t first = std::min<uint32_t>(o->gb_land_rows, kGroupRowsFirstCopy);
-    MGV_CUDA_TRY(cudaMemcpyAsync(h + 16, o->gb_dev_rows, sizeof(mgv_group_row) * (size_t)first,
-                                 cudaMemcpyDeviceToHost, s));
+    const uint32_t cap = o->gtab.cap;
+    const bool sort = !o->gb_unordered && cap <= kDeviceOrderCap && o->gb.max_groups > kHostOrderGroups;
+    const bool direct = !sort && cap + 1 <= o->gb_land_rows;  // packed rows straight into the landing zone
+    o->gb_clean = false;
+    if (cap <= kSmallGroupCap) {
+        MGV_CUDA_TRY(launch_group_close(o->gtab, o->gb_land_dev, sort, s, ctx));
+    } else if (sort) {
+        MGV_CUDA_TRY(launch_group_pack(o->gtab, o->gb_dev_rows, o->gb_dev_count, nullptr, s, ctx));
+        const GroupSortJob job{o->gb_dev_rows, o->gb_dev_count, o->gb_pairs, o->gb_land_dev->rows,
+                               o->gb_dev_more, o->gb_land_dev, nullptr, cap + 1, o->gb_land_rows};
+        MGV_CUDA_TRY(launch_group_sort(nullptr, job, 1, s, ctx));
+    } else {
+        MGV_CUDA_TRY(launch_group_pack(o->gtab, direct ? o->gb_land_dev->rows : o->gb_dev_rows, o->gb_dev_count,
+                                       o->gb_land_dev, s, ctx));
+    }
     MGV_CUDA_TRY(cudaStreamSynchronize(s));
-    const uint32_t w[2] = {reinterpret_cast<uint32_t*>(h)[0], reinterpret_cast<uint32_t*>(h)[1]};
+    o->gb_clean = true;
+    const GroupLanding* L = o->gb_land;
+    const uint32_t w[2] = {L->err[0], L->err[1]};
     mgv_status st = report_device_error(ctx, w, s);
     if (st != MGV_OK) return st;
-    uint32_t n = 0;
-    std::memcpy(&n, h + 8, sizeof(n));
-    const mgv_group_row* rows = reinterpret_cast<const mgv_group_row*>(h + 16);
-    o->gb_rows.assign(rows, rows + std::min(n, first));
-    if (n > first) {  // the rest, through the landing zone while it holds them
+    const uint32_t n = L->count;
+    o->gb_n = n;
+    o->gb_sorted = sort;
+    o->gb_view = L->rows;
+    if (cap > kSmallGroupCap && !sort && !direct && n <= o->gb_land_rows) {
+        MGV_CUDA_TRY(cudaMemcpyAsync(o->gb_land->rows, o->gb_dev_rows, sizeof(mgv_group_row) * (size_t)n,
+                                     cudaMemcpyDeviceToHost, s));
+        MGV_CUDA_TRY(cudaStreamSynchronize(s));
+    } else if (n > o->gb_land_rows) {  // more rows than the landing zone holds
+        const uint32_t landed = sort ? o->gb_land_rows : 0;
         o->gb_rows.resize(n);
-        const uint32_t land_more = std::min(n, o->gb_land_rows) - first;
-        if (land_more) {
-            MGV_CUDA_TRY(cudaMemcpyAsync(h + 16, o->gb_dev_rows + first, sizeof(mgv_group_row) * (size_t)land_more,
-                                         cudaMemcpyDeviceToHost, s));
-            MGV_CUDA_TRY(cudaStreamSynchronize(s));
-            std::memcpy(o->gb_rows.data() + first, h + 16, sizeof(mgv_group_row) * (size_t)land_more);
-        }
-        if (n > o->gb_land_rows)
-            MGV_CUDA_TRY(cudaMemcpy(o->gb_rows.data() + o->gb_land_rows, o->gb_dev_rows + o->gb_land_rows,
-                                    sizeof(mgv_group_row) * (size_t)(n - o->gb_land_rows), cudaMemcpyDeviceToHost));
+        std::copy(L->rows, L->rows + landed, o->gb_rows.begin());
+        MGV_CUDA_TRY(cudaMemcpyAsync(o->gb_rows.data() + landed, sort ? o->gb_dev_more : o->gb_dev_rows,
+                                     sizeof(mgv_group_row) * (size_t)(n - landed), cudaMemcpyDeviceToHost, s));
+        MGV_CUDA_TRY(cudaStreamSynchronize(s));
+        o->gb_view = o->gb_rows.data();
     }
-    o->gb_sorted = false;  // ordered by group when first read (mgv_op_result)
     return MGV_OK;
 }
 
@@ -205,6 +216,7 @@ mgv_status mgv_ctx_create(int device, mgv_ctx** out) {
     if (e == cudaSuccess) e = cudaMalloc(&c->d_err, 2 * sizeof(uint32_t));
     if (e == cudaSuccess) e = cudaMemset(c->d_err, 0, 2 * sizeof(uint32_t));
     if (e == cudaSuccess) e = cudaMallocHost(&c->h_stage, 8 * sizeof(unsigned long long));
+    if (e == cudaSuccess) e = group_rows_init();
     if (e != cudaSuccess) {
         if (c->h_stage) cudaFreeHost(c->h_stage);
         if (c->d_err) cudaFree(c->d_err);
@@ -582,13 +594,24 @@ mgv_status mgv_op_create_groupby(mgv_ctx* ctx, const mgv_groupby_desc* d, mgv_op
     if (st == MGV_OK) st = dev_alloc(o, (void**)&g.sums, sizeof(unsigned long long) * cap);
     if (st == MGV_OK) st = dev_alloc(o, (void**)&g.counts, sizeof(unsigned long long) * cap);
     if (st == MGV_OK) st = dev_alloc(o, (void**)&g.special, 2 * sizeof(unsigned long long));
-    if (st == MGV_OK) st = dev_alloc(o, (void**)&o->gb_dev_rows, sizeof(mgv_group_row) * ((size_t)cap + 1));
-    if (st == MGV_OK) st = dev_alloc(o, (void**)&o->gb_dev_count, sizeof(uint32_t));
-    // pinned landing zone: results of up to 64 Ki groups come back with one synchronisation
+    if (st == MGV_OK) st = dev_alloc(o, (void**)&o->gb_dev_count, 2 * sizeof(uint32_t));
+    // landing zone: a larger result's further rows are copied after it
     o->gb_land_rows = std::min<uint32_t>(cap + 1, 1u << 16);
-    if (st == MGV_OK &&
-        cudaMallocHost(&o->gb_land, 16 + sizeof(mgv_group_row) * (size_t)o->gb_land_rows) != cudaSuccess)
-        st = fail(MGV_ENOMEM, "pinned host allocation");
+    if (cap > kSmallGroupCap) {
+        if (st == MGV_OK) st = dev_alloc(o, (void**)&o->gb_dev_rows, sizeof(mgv_group_row) * ((size_t)cap + 1));
+        if (st == MGV_OK && cap <= kDeviceOrderCap)
+            st = dev_alloc(o, (void**)&o->gb_pairs, 2 * sizeof(unsigned long long) * ((size_t)cap + 1));
+        if (st == MGV_OK && cap <= kDeviceOrderCap && cap + 1 > o->gb_land_rows)
+            st = dev_alloc(o, (void**)&o->gb_dev_more, sizeof(mgv_group_row) * ((size_t)cap + 1 - o->gb_land_rows));
+    }
+    if (st == MGV_OK) {
+        cudaError_t e = cudaMallocHost(&o->gb_land, sizeof(GroupLanding) + sizeof(mgv_group_row) * (size_t)o->gb_land_rows);
+        if (e == cudaSuccess) e = cudaHostGetDevicePointer(reinterpret_cast<void**>(&o->gb_land_dev), o->gb_land, 0);
+        if (e != cudaSuccess) {
+            if (o->gb_land) cudaFreeHost(o->gb_land);
+            st = fail(MGV_ENOMEM, "pinned host allocation");
+        }
+    }
     if (st != MGV_OK) {
         for (void* p : o->allocs) cudaFree(p);
         delete o;
@@ -713,10 +736,10 @@ static mgv_status op_reset(Op* o, cudaStream_t s) {
                 return fail(MGV_ESTATE, "hash_probe opened before its build side was closed");
             break;
         case OpKind::Groupby:
-            MGV_CUDA_TRY(launch_fill_i32(o->gtab.keys, o->gtab.cap, kEmptyKey, s, o->ctx));
-            MGV_CUDA_TRY(cudaMemsetAsync(o->gtab.sums, 0, sizeof(unsigned long long) * o->gtab.cap, s));
-            MGV_CUDA_TRY(cudaMemsetAsync(o->gtab.counts, 0, sizeof(unsigned long long) * o->gtab.cap, s));
-            MGV_CUDA_TRY(cudaMemsetAsync(o->gtab.special, 0, 2 * sizeof(unsigned long long), s));
+            if (!o->gb_clean) MGV_CUDA_TRY(launch_group_reset(o->gtab, o->gb_dev_count, s, o->ctx));
+            o->gb_clean = true;  // until a consume or a close touches it
+            o->gb_view = nullptr;
+            o->gb_n = 0;
             o->gb_rows.clear();
             break;
         case OpKind::Partition:
@@ -887,11 +910,13 @@ mgv_status mgv_op_result(mgv_op* o, void* out, size_t bytes, size_t* needed) {
         case OpKind::Sink: src = &o->sink_rows; n = sizeof(o->sink_rows); break;
         case OpKind::Groupby:
             if (!o->gb_sorted) {
+                if (o->gb_view != o->gb_rows.data()) o->gb_rows.assign(o->gb_view, o->gb_view + o->gb_n);
                 sort_group_rows(o->gb_rows);
+                o->gb_view = o->gb_rows.data();
                 o->gb_sorted = true;
             }
-            src = o->gb_rows.data();
-            n = o->gb_rows.size() * sizeof(mgv_group_row);
+            src = o->gb_view;
+            n = o->gb_n * sizeof(mgv_group_row);
             break;
         case OpKind::Partition:
             if (!o->pt_hist_valid) {  // the rows per partition, read once after the close's stream
@@ -1098,6 +1123,7 @@ static mgv_status consume_cols(Op* head, const int32_t* const* cols, uint32_t nc
             const int32_t g = (int32_t)term->gb.group_col, v = term->gb.value_col;
             if (!ref_ok(g) || g == -1 || !ref_ok(v)) return fail(MGV_EINVAL, "group-by column not in input");
             if (n == 0) return MGV_OK;
+            term->gb_clean = false;
             a.term = kTermGroupby;
             a.ref[0] = g;
             a.ref[1] = v;

@@ -928,41 +928,6 @@ __global__ void k_batch_compact(const BatchOut* __restrict__ outs, const BatchIt
     }
 }
 
-// Packs the non-empty groups of a global group table (the group INT32_MIN
-// included) into out[0 .. *count); one warp-aggregated reservation per warp.
-__global__ void k_group_pack(GroupTableView gt, mgv_group_row* __restrict__ out, uint32_t* count) {
-    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-    const uint64_t end = ((uint64_t)gt.cap + 1 + 31) & ~31ull;  // whole warps take part in the ballots
-    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < end; i += stride) {
-        const bool special = i == gt.cap;
-        bool keep = false;
-        mgv_group_row r{};
-        if (i <= gt.cap) {
-            r.group = special ? kEmptyKey : gt.keys[i];
-            const unsigned long long c = special ? gt.special[1] : gt.counts[i];
-            keep = c != 0 && (special || r.group != kEmptyKey);
-            if (keep) {
-                r.sum = (int64_t)(special ? gt.special[0] : gt.sums[i]);
-                r.count = (int64_t)c;
-            }
-        }
-        const unsigned m = __ballot_sync(0xffffffffu, keep);
-        uint32_t base = 0;
-        if (lane_id() == 0 && m) base = atomicAdd(count, (uint32_t)__popc(m));
-        base = __shfl_sync(0xffffffffu, base, 0);
-        if (keep) out[base + __popc(m & ((1u << lane_id()) - 1u))] = r;
-    }
-}
-
-cudaError_t launch_group_pack(const GroupTableView& gt, mgv_group_row* out, uint32_t* count, cudaStream_t s,
-                              Context* ctx) {
-    const uint64_t want = ((uint64_t)gt.cap + 1 + 255) / 256;
-    const uint64_t cap = (uint64_t)ctx->prop.multiProcessorCount * 8;
-    k_group_pack<<<(int)(want < cap ? want : cap), 256, 0, s>>>(gt, out, count);
-    ctx->launches++;
-    return cudaGetLastError();
-}
-
 cudaError_t launch_batch(const ChainDev* d_qs, const BatchOut* d_outs, const BatchItem* probe_items, uint32_t n_probe,
                          const BatchItem* compact_items, uint32_t n_compact, int ctas_per_sm, uint32_t item_order,
                          cudaStream_t s, Context* ctx) {

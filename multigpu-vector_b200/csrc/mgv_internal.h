@@ -162,11 +162,18 @@ struct Op {
     // group-by
     mgv_groupby_desc gb{};
     GroupTableView gtab{};
-    std::vector<mgv_group_row> gb_rows;
-    bool gb_sorted = false;  // gb_rows ordered by group (done at the first result read)
-    mgv_group_row* gb_dev_rows = nullptr;  // [cap + 1] packed by close()
-    uint32_t* gb_dev_count = nullptr;
-    unsigned char* gb_land = nullptr;      // pinned: {err[2], count, pad} then kGroupLandRows rows
+    const mgv_group_row* gb_view = nullptr;  // the closed result's rows: in the landing zone or gb_rows
+    uint32_t gb_n = 0;
+    std::vector<mgv_group_row> gb_rows;      // rows the landing zone does not hold, or ordered on the host
+    bool gb_sorted = false;                  // gb_view is ordered by group (else done at the first result read)
+    bool gb_unordered = false;               // nobody asks for an order: close leaves the rows as they come
+    bool gb_clean = false;                   // the table is empty on the device (a close leaves it so)
+    mgv_group_row* gb_dev_rows = nullptr;    // [cap + 1] packed by the close of a large table
+    uint32_t* gb_dev_count = nullptr;        // {groups packed, CTAs done}
+    unsigned long long* gb_pairs = nullptr;  // sorting space of a large table
+    mgv_group_row* gb_dev_more = nullptr;    // ordered rows past the landing zone
+    struct GroupLanding* gb_land = nullptr;  // pinned, mapped: gb_land_rows rows
+    struct GroupLanding* gb_land_dev = nullptr;
     uint32_t gb_land_rows = 0;
     // partition
     mgv_partition_desc pt{};
@@ -370,7 +377,33 @@ struct BatchOut {  // packed result region of a query
     uint32_t capacity;
     uint32_t pad;
 };
-cudaError_t launch_group_pack(const GroupTableView& gt, mgv_group_row* out, uint32_t* count, cudaStream_t s,
+// A group-by operator's landing zone in pinned, mapped host memory.
+struct GroupLanding {
+    uint32_t err[2];
+    uint32_t count;
+    uint32_t pad;
+    mgv_group_row rows[1];
+};
+// Packed rows to be ordered by group (group_rows.cu).
+struct GroupSortJob {
+    const mgv_group_row* rows;
+    uint32_t* count;            // rows found (may exceed capacity: then an error is set)
+    unsigned long long* pairs;  // 2 * capacity, used when the rows do not fit shared memory
+    mgv_group_row* out;         // the first out_rows rows
+    mgv_group_row* more;        // the rows past them
+    GroupLanding* land;         // nullable: header to fill in
+    uint32_t* host_count;       // nullable
+    uint32_t capacity;
+    uint32_t out_rows;
+};
+constexpr uint32_t kSmallGroupCap = 8192;      // slots of a table that one CTA closes
+constexpr uint32_t kDeviceOrderCap = 1u << 21;  // slots of the largest table ordered on the device
+cudaError_t group_rows_init();  // once per device: the kernels' shared memory limits
+cudaError_t launch_group_reset(const GroupTableView& gt, uint32_t* count, cudaStream_t s, Context* ctx);
+cudaError_t launch_group_close(const GroupTableView& gt, GroupLanding* land, bool sort, cudaStream_t s, Context* ctx);
+cudaError_t launch_group_pack(const GroupTableView& gt, mgv_group_row* rows, uint32_t* count, GroupLanding* land,
+                              cudaStream_t s, Context* ctx);
+cudaError_t launch_group_sort(const GroupSortJob* d_jobs, const GroupSortJob& job0, uint32_t njobs, cudaStream_t s,
                               Context* ctx);
 cudaError_t launch_batch(const ChainDev* d_qs, const BatchOut* d_outs, const BatchItem* probe_items, uint32_t n_probe,
                          const BatchItem* compact_items, uint32_t n_compact, int ctas_per_sm, uint32_t item_order,

@@ -492,7 +492,10 @@ mgv_status plain_groupby(mgv_server* S, uint32_t max_groups, mgv_op** out) {
     }
     mgv_groupby_desc gd{2, 3, c, 0};
     mgv_status st = mgv_op_create_groupby(S->ctx, &gd, out);
-    if (st == MGV_OK) S->plain_gb[c] = *out;
+    if (st == MGV_OK) {
+        (*out)->gb_unordered = true;
+        S->plain_gb[c] = *out;
+    }
     return st;
 }
 
@@ -511,7 +514,10 @@ mgv_status run_plain(mgv_server* S, Request& q) {
     if (st == MGV_OK) st = mgv_op_open(sel, nullptr);
     if (st == MGV_OK) st = mgv_op_consume_columns(sel, cols, 4, r.probe_rows, nullptr);
     if (st == MGV_OK) st = mgv_op_close(sel, nullptr);
-    if (st == MGV_OK) q.rows = static_cast<Op*>(gb)->gb_rows;  // in no particular order, as the batched server's
+    if (st == MGV_OK) {  // in no particular order, as the batched server's
+        const Op* g = static_cast<Op*>(gb);
+        q.rows.assign(g->gb_view, g->gb_view + g->gb_n);
+    }
     mgv_op_destroy(sel);
     mgv_op_destroy(probe);
     return st;
@@ -646,12 +652,6 @@ mgv_status mgv_server_create(mgv_ctx* ctx, const mgv_server_config* cfg, mgv_ser
             delete S;
             return st;
         }
-        // the host rows of the class's largest result, written once now: the
-        // first request of a class then finds its pages present instead of
-        // faulting them in (a tenth of a millisecond for 65536 groups)
-        std::vector<mgv_group_row>& rows = static_cast<Op*>(gb)->gb_rows;
-        rows.resize(c);
-        rows.clear();
     }
     // landing zones pinned up front (four per in-flight slot, at most eight),
     // so serving rarely pins (slow) while batches are in flight and waiters

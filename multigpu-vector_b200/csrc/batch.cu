@@ -55,7 +55,7 @@ struct mgv_batch {
     BatchItem* d_compact_items = nullptr;
     uint32_t n_build = 0, n_probe = 0, n_compact = 0;
     GroupSortJob* d_sorts = nullptr;  // queries whose groups are ordered on the device, largest first
-    uint32_t n_sorts = 0;
+    uint32_t n_sorts = 0, max_sort_rows = 0;
     std::vector<uint8_t> ordered;  // per query: its landed rows are in group order
     std::vector<uint64_t> out_offset;  // first packed row of each query
     // host landing zone: each query's rows are written straight into it (pinned,
@@ -116,9 +116,10 @@ mgv_status enqueue_run(mgv_batch* b, cudaStream_t s) {
     layout.t.key_only = b->key_only;
     MGV_CUDA_TRY(launch_build_regions(b->d_jobs, layout, (uint32_t)b->q.size(), b->d_build_items, b->n_build, 0, 0,
                                       b->total_regions, b->max_job_regions, b->rsc, true, false, s, ctx));
-    MGV_CUDA_TRY(launch_batch(b->d_qs, b->d_outs, b->d_probe_items, b->n_probe, b->d_compact_items, b->n_compact,
-                              (int)b->cfg.probe_ctas_per_sm, b->cfg.item_order, s, ctx));
-    MGV_CUDA_TRY(launch_group_sort(b->d_sorts, GroupSortJob{}, b->n_sorts, s, ctx));
+    MGV_CUDA_TRY(launch_batch(b->d_qs, b->d_probe_items, b->n_probe, (int)b->cfg.probe_ctas_per_sm, b->cfg.item_order,
+                              s, ctx));
+    MGV_CUDA_TRY(launch_batch_compact(b->d_outs, b->d_compact_items, b->n_compact, s, ctx));
+    MGV_CUDA_TRY(launch_group_sort(b->d_sorts, GroupSortJob{}, b->n_sorts, b->max_sort_rows, s, ctx));
     MGV_CUDA_TRY(cudaMemcpyAsync(b->h_counts, b->out_counts, sizeof(uint32_t) * b->q.size(), cudaMemcpyDeviceToHost, s));
     MGV_CUDA_TRY(cudaMemcpyAsync(b->h_err, ctx->d_err, 2 * sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
     return MGV_OK;
@@ -137,7 +138,7 @@ mgv_status check_run(mgv_batch* b) {
 void sort_rows(std::vector<mgv_group_row>& v) { sort_group_rows(v); }
 
 // Groups up to this many per query are ordered on the device when a batch has
-// the memory for it (40 bytes of packed rows and sorting space per group).
+// the memory for it (44 bytes of packed rows and sorting space per group).
 constexpr uint32_t kDeviceOrderGroups = kDeviceOrderCap / 2;
 
 mgv_status create_batch(mgv_ctx* ctx, const mgv_query_desc* qs, uint32_t nq, const mgv_batch_config* config,
@@ -239,7 +240,7 @@ mgv_status create_batch(mgv_ctx* ctx, const mgv_query_desc* qs, uint32_t nq, con
         b->ordered[i] = 1;
         sorts.push_back(i);
         rows_off[i] = take(sizeof(mgv_group_row) * (size_t)qs[i].max_groups);
-        pairs_off[i] = take(2 * sizeof(unsigned long long) * (size_t)qs[i].max_groups);
+        pairs_off[i] = take((2 * sizeof(unsigned long long) + sizeof(uint32_t)) * (size_t)qs[i].max_groups);
     }
     std::stable_sort(sorts.begin(), sorts.end(),
                      [&](uint32_t x, uint32_t y) { return qs[x].max_groups > qs[y].max_groups; });
@@ -251,8 +252,8 @@ mgv_status create_batch(mgv_ctx* ctx, const mgv_query_desc* qs, uint32_t nq, con
             bi.push_back(BatchItem{i, 0, lo, std::min<uint64_t>(qs[i].build_rows, lo + cfg.build_item_rows)});
         for (uint64_t lo = 0; lo < qs[i].probe_rows; lo += cfg.probe_item_rows)
             pi.push_back(BatchItem{i, 0, lo, std::min<uint64_t>(qs[i].probe_rows, lo + cfg.probe_item_rows)});
-        for (uint64_t lo = 0; lo <= gcap[i]; lo += 65536)
-            ci.push_back(BatchItem{i, 0, lo, std::min<uint64_t>((uint64_t)gcap[i] + 1, lo + 65536)});
+        for (uint64_t lo = 0; lo <= gcap[i]; lo += kCompactSlots)
+            ci.push_back(BatchItem{i, 0, lo, std::min<uint64_t>((uint64_t)gcap[i] + 1, lo + kCompactSlots)});
     }
     const size_t bi_off = take(sizeof(BatchItem) * std::max<size_t>(bi.size(), 1));
     const size_t pi_off = take(sizeof(BatchItem) * std::max<size_t>(pi.size(), 1));
@@ -345,10 +346,17 @@ mgv_status create_batch(mgv_ctx* ctx, const mgv_query_desc* qs, uint32_t nq, con
         ho[i] = BatchOut{g, packed, b->out_counts + i, qs[i].max_groups, 0};
     }
     std::vector<GroupSortJob> hs;
-    for (uint32_t i : sorts)
-        hs.push_back(GroupSortJob{ho[i].rows, b->out_counts + i, reinterpret_cast<unsigned long long*>(A + pairs_off[i]),
-                                  b->h_rows_dev + b->out_offset[i], nullptr, nullptr, nullptr, qs[i].max_groups,
-                                  qs[i].max_groups});
+    for (uint32_t i : sorts) {
+        GroupSortJob j{};
+        j.rows = ho[i].rows;
+        j.count = j.found = b->out_counts + i;
+        j.pairs = reinterpret_cast<unsigned long long*>(A + pairs_off[i]);
+        j.order = reinterpret_cast<uint32_t*>(j.pairs + 2 * (size_t)qs[i].max_groups);
+        j.out = b->h_rows_dev + b->out_offset[i];
+        j.capacity = j.out_rows = qs[i].max_groups;
+        b->max_sort_rows = std::max(b->max_sort_rows, qs[i].max_groups);
+        hs.push_back(j);
+    }
     b->d_sorts = reinterpret_cast<GroupSortJob*>(A + sorts_off);
     b->n_sorts = (uint32_t)hs.size();
     e = cudaMemcpy(b->d_qs, hq.data(), sizeof(ChainDev) * nq, cudaMemcpyHostToDevice);

@@ -116,8 +116,8 @@ void sort_group_rows(std::vector<mgv_group_row>& v) {
 // and their count; one synchronisation.  The kernels leave the table empty, so
 // the next open has nothing to clear.  A table of up to kSmallGroupCap slots
 // takes one kernel of one CTA (a table that size is read in a few
-// microseconds); a larger one is packed by the whole GPU and ordered by one
-// CTA; one past kDeviceOrderCap slots (half a GiB of sorting space and up) is
+// microseconds); a larger one is packed by the whole GPU, ordered by one CTA
+// and written out by many; one past kDeviceOrderCap slots (half a GiB of sorting space and up) is
 // ordered by the host when its result is read, and so is one of at most
 // kHostOrderGroups groups (a microsecond on the host).
 constexpr uint32_t kHostOrderGroups = 64;
@@ -132,9 +132,18 @@ static mgv_status close_groupby(Op* o, cudaStream_t s) {
         MGV_CUDA_TRY(launch_group_close(o->gtab, o->gb_land_dev, sort, s, ctx));
     } else if (sort) {
         MGV_CUDA_TRY(launch_group_pack(o->gtab, o->gb_dev_rows, o->gb_dev_count, nullptr, s, ctx));
-        const GroupSortJob job{o->gb_dev_rows, o->gb_dev_count, o->gb_pairs, o->gb_land_dev->rows,
-                               o->gb_dev_more, o->gb_land_dev, nullptr, cap + 1, o->gb_land_rows};
-        MGV_CUDA_TRY(launch_group_sort(nullptr, job, 1, s, ctx));
+        GroupSortJob job{};
+        job.rows = o->gb_dev_rows;
+        job.count = o->gb_dev_count;
+        job.found = o->gb_dev_count + 2;
+        job.pairs = o->gb_pairs;
+        job.order = reinterpret_cast<uint32_t*>(o->gb_pairs + 2 * ((size_t)cap + 1));
+        job.out = o->gb_land_dev->rows;
+        job.more = o->gb_dev_more;
+        job.land = o->gb_land_dev;
+        job.capacity = cap + 1;
+        job.out_rows = o->gb_land_rows;
+        MGV_CUDA_TRY(launch_group_sort(nullptr, job, 1, cap + 1, s, ctx));
     } else {
         MGV_CUDA_TRY(launch_group_pack(o->gtab, direct ? o->gb_land_dev->rows : o->gb_dev_rows, o->gb_dev_count,
                                        o->gb_land_dev, s, ctx));
@@ -594,13 +603,13 @@ mgv_status mgv_op_create_groupby(mgv_ctx* ctx, const mgv_groupby_desc* d, mgv_op
     if (st == MGV_OK) st = dev_alloc(o, (void**)&g.sums, sizeof(unsigned long long) * cap);
     if (st == MGV_OK) st = dev_alloc(o, (void**)&g.counts, sizeof(unsigned long long) * cap);
     if (st == MGV_OK) st = dev_alloc(o, (void**)&g.special, 2 * sizeof(unsigned long long));
-    if (st == MGV_OK) st = dev_alloc(o, (void**)&o->gb_dev_count, 2 * sizeof(uint32_t));
+    if (st == MGV_OK) st = dev_alloc(o, (void**)&o->gb_dev_count, 3 * sizeof(uint32_t));
     // landing zone: a larger result's further rows are copied after it
     o->gb_land_rows = std::min<uint32_t>(cap + 1, 1u << 16);
     if (cap > kSmallGroupCap) {
         if (st == MGV_OK) st = dev_alloc(o, (void**)&o->gb_dev_rows, sizeof(mgv_group_row) * ((size_t)cap + 1));
         if (st == MGV_OK && cap <= kDeviceOrderCap)
-            st = dev_alloc(o, (void**)&o->gb_pairs, 2 * sizeof(unsigned long long) * ((size_t)cap + 1));
+            st = dev_alloc(o, (void**)&o->gb_pairs, (2 * sizeof(unsigned long long) + sizeof(uint32_t)) * ((size_t)cap + 1));
         if (st == MGV_OK && cap <= kDeviceOrderCap && cap + 1 > o->gb_land_rows)
             st = dev_alloc(o, (void**)&o->gb_dev_more, sizeof(mgv_group_row) * ((size_t)cap + 1 - o->gb_land_rows));
     }

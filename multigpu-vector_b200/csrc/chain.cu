@@ -888,71 +888,20 @@ cudaError_t launch_cells_prefix(const CellsView& c, cudaStream_t s, Context* ctx
     return cudaGetLastError();
 }
 
-// Packs each query's groups into its output region (unsorted) and counts them;
-// one warp-aggregated reservation of output rows per warp (a query's counter
-// is one address, and per-row atomics on it serialise in L2).
-__global__ void k_batch_compact(const BatchOut* __restrict__ outs, const BatchItem* __restrict__ items,
-                                uint32_t nitems, uint32_t* err) {
-    const uint32_t lane = lane_id();
-    for (uint32_t it = blockIdx.x; it < nitems; it += gridDim.x) {
-        const BatchItem item = items[it];
-        const BatchOut& o = outs[item.q];
-        // whole warps take part in the ballots
-        const uint64_t end = item.lo + ((item.hi - item.lo + 31) & ~31ull);
-        for (uint64_t i = item.lo + threadIdx.x; i < end; i += blockDim.x) {
-            bool keep = false;
-            mgv_group_row r{};
-            if (i < item.hi) {
-                const bool special = i == o.gt.cap;  // one extra index for the group INT32_MIN
-                const int32_t k = special ? kEmptyKey : o.gt.keys[i];
-                const unsigned long long c = special ? o.gt.special[1] : o.gt.counts[i];
-                keep = (special || k != kEmptyKey) && c != 0;
-                if (keep) {
-                    r.group = k;
-                    r.sum = (int64_t)(special ? o.gt.special[0] : o.gt.sums[i]);
-                    r.count = (int64_t)c;
-                }
-            }
-            const unsigned m = __ballot_sync(0xffffffffu, keep);
-            uint32_t base = 0;
-            if (lane == 0 && m) base = atomicAdd(o.count, (uint32_t)__popc(m));
-            base = __shfl_sync(0xffffffffu, base, 0);
-            if (!keep) continue;
-            const uint32_t pos = base + __popc(m & ((1u << lane) - 1u));
-            if (pos >= o.capacity) {
-                set_error(err, kDevOverflow, 30);
-                continue;
-            }
-            o.rows[pos] = r;
-        }
-    }
-}
-
-cudaError_t launch_batch(const ChainDev* d_qs, const BatchOut* d_outs, const BatchItem* probe_items, uint32_t n_probe,
-                         const BatchItem* compact_items, uint32_t n_compact, int ctas_per_sm, uint32_t item_order,
-                         cudaStream_t s, Context* ctx) {
-    const int sms = ctx->prop.multiProcessorCount;
-    if (n_probe) {
-        const size_t smem = kRingBytes + smem_groups_bytes(kMaxSmemGroups);
-        cudaError_t e = cudaFuncSetAttribute(k_batch_probe, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return e;
-        int per_sm = 0;
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_batch_probe, kChainBlock, smem);
-        per_sm = std::max(per_sm, 1);
-        if (ctas_per_sm > 0 && ctas_per_sm < per_sm) per_sm = ctas_per_sm;
-        const int grid = (int)std::min<uint64_t>((uint64_t)per_sm * sms, n_probe);
-        k_batch_probe<<<grid, kChainBlock, smem, s>>>(d_qs, probe_items, n_probe, item_order, ctx->d_err);
-        ctx->launches++;
-        e = cudaGetLastError();
-        if (e != cudaSuccess) return e;
-    }
-    if (n_compact) {
-        const int grid = (int)std::min<uint64_t>((uint64_t)sms * 8, n_compact);
-        k_batch_compact<<<grid, 256, 0, s>>>(d_outs, compact_items, n_compact, ctx->d_err);
-        ctx->launches++;
-        return cudaGetLastError();
-    }
-    return cudaSuccess;
+cudaError_t launch_batch(const ChainDev* d_qs, const BatchItem* probe_items, uint32_t n_probe, int ctas_per_sm,
+                         uint32_t item_order, cudaStream_t s, Context* ctx) {
+    if (n_probe == 0) return cudaSuccess;
+    const size_t smem = kRingBytes + smem_groups_bytes(kMaxSmemGroups);
+    cudaError_t e = cudaFuncSetAttribute(k_batch_probe, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    int per_sm = 0;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_batch_probe, kChainBlock, smem);
+    per_sm = std::max(per_sm, 1);
+    if (ctas_per_sm > 0 && ctas_per_sm < per_sm) per_sm = ctas_per_sm;
+    const int grid = (int)std::min<uint64_t>((uint64_t)per_sm * ctx->prop.multiProcessorCount, n_probe);
+    k_batch_probe<<<grid, kChainBlock, smem, s>>>(d_qs, probe_items, n_probe, item_order, ctx->d_err);
+    ctx->launches++;
+    return cudaGetLastError();
 }
 
 template <bool SEL, bool PROBE, int TERM>

@@ -169,8 +169,8 @@ struct Op {
     bool gb_unordered = false;               // nobody asks for an order: close leaves the rows as they come
     bool gb_clean = false;                   // the table is empty on the device (a close leaves it so)
     mgv_group_row* gb_dev_rows = nullptr;    // [cap + 1] packed by the close of a large table
-    uint32_t* gb_dev_count = nullptr;        // {groups packed, CTAs done}
-    unsigned long long* gb_pairs = nullptr;  // sorting space of a large table
+    uint32_t* gb_dev_count = nullptr;        // {groups packed, CTAs done, groups found}
+    unsigned long long* gb_pairs = nullptr;  // sorting space of a large table: pairs, then the order
     mgv_group_row* gb_dev_more = nullptr;    // ordered rows past the landing zone
     struct GroupLanding* gb_land = nullptr;  // pinned, mapped: gb_land_rows rows
     struct GroupLanding* gb_land_dev = nullptr;
@@ -388,26 +388,32 @@ struct GroupLanding {
 struct GroupSortJob {
     const mgv_group_row* rows;
     uint32_t* count;            // rows found (may exceed capacity: then an error is set)
+    uint32_t* found;            // the same, kept for the writing of the rows
     unsigned long long* pairs;  // 2 * capacity, used when the rows do not fit shared memory
+    uint32_t* order;            // capacity
     mgv_group_row* out;         // the first out_rows rows
     mgv_group_row* more;        // the rows past them
     GroupLanding* land;         // nullable: header to fill in
-    uint32_t* host_count;       // nullable
     uint32_t capacity;
     uint32_t out_rows;
 };
-constexpr uint32_t kSmallGroupCap = 8192;      // slots of a table that one CTA closes
+constexpr uint32_t kSmallGroupCap = 2048;      // slots of a table that one CTA closes
 constexpr uint32_t kDeviceOrderCap = 1u << 21;  // slots of the largest table ordered on the device
 cudaError_t group_rows_init();  // once per device: the kernels' shared memory limits
 cudaError_t launch_group_reset(const GroupTableView& gt, uint32_t* count, cudaStream_t s, Context* ctx);
 cudaError_t launch_group_close(const GroupTableView& gt, GroupLanding* land, bool sort, cudaStream_t s, Context* ctx);
 cudaError_t launch_group_pack(const GroupTableView& gt, mgv_group_row* rows, uint32_t* count, GroupLanding* land,
                               cudaStream_t s, Context* ctx);
-cudaError_t launch_group_sort(const GroupSortJob* d_jobs, const GroupSortJob& job0, uint32_t njobs, cudaStream_t s,
-                              Context* ctx);
-cudaError_t launch_batch(const ChainDev* d_qs, const BatchOut* d_outs, const BatchItem* probe_items, uint32_t n_probe,
-                         const BatchItem* compact_items, uint32_t n_compact, int ctas_per_sm, uint32_t item_order,
-                         cudaStream_t s, Context* ctx);
+// Orders the jobs' rows (max_rows: the largest capacity) and writes them out.
+cudaError_t launch_group_sort(const GroupSortJob* d_jobs, const GroupSortJob& job0, uint32_t njobs, uint32_t max_rows,
+                              cudaStream_t s, Context* ctx);
+cudaError_t launch_batch(const ChainDev* d_qs, const BatchItem* probe_items, uint32_t n_probe, int ctas_per_sm,
+                         uint32_t item_order, cudaStream_t s, Context* ctx);
+// Packs the groups of many tables (items: slots [lo, hi) of query q, at most
+// kCompactSlots each) into their output regions.
+constexpr uint64_t kCompactSlots = 4096;
+cudaError_t launch_batch_compact(const BatchOut* d_outs, const BatchItem* items, uint32_t nitems, cudaStream_t s,
+                                 Context* ctx);
 // Shared scans: the persistent probe -> cells kernel over (scan, rows)
 // items (rows per item < 2^kCellRowBits), then the prefix over each scan's
 // ranges (`scans` are host-side copies of the device descriptors' cells).

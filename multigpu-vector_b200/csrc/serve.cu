@@ -290,8 +290,8 @@ mgv_status launch(mgv_server* S, Inflight& sl) {
         if (scan_of[i] < 0)
             for (uint64_t lo = 0; lo < sl.reqs[i]->r.probe_rows; lo += item_rows)
                 pi.push_back(BatchItem{i, 0, lo, std::min<uint64_t>(sl.reqs[i]->r.probe_rows, lo + item_rows)});
-        for (uint64_t lo = 0; lo <= caps[i]; lo += 65536)
-            ci.push_back(BatchItem{i, 0, lo, std::min<uint64_t>((uint64_t)caps[i] + 1, lo + 65536)});
+        for (uint64_t lo = 0; lo <= caps[i]; lo += kCompactSlots)
+            ci.push_back(BatchItem{i, 0, lo, std::min<uint64_t>((uint64_t)caps[i] + 1, lo + kCompactSlots)});
     }
     for (uint32_t g = 0; g < (uint32_t)scans.size(); ++g) {
         const uint64_t n = sl.reqs[scans[g].reqs[0]]->r.probe_rows;
@@ -418,16 +418,15 @@ mgv_status launch(mgv_server* S, Inflight& sl) {
     MGV_CUDA_TRY(launch_fill_i32(reinterpret_cast<int32_t*>(A), slots, kEmptyKey, s, ctx));
     MGV_CUDA_TRY(cudaMemsetAsync(A + zero_begin, 0, zero_end - zero_begin, s));
     MGV_CUDA_TRY(cudaMemsetAsync(A + counts_off, 0, 4ull * nq, s));
-    MGV_CUDA_TRY(launch_batch(reinterpret_cast<ChainDev*>(A + qs_off), reinterpret_cast<BatchOut*>(A + outs_off),
-                              reinterpret_cast<BatchItem*>(A + pi_off), (uint32_t)pi.size(), nullptr, 0u, 0, 0u,
-                              s, ctx));
+    MGV_CUDA_TRY(launch_batch(reinterpret_cast<ChainDev*>(A + qs_off), reinterpret_cast<BatchItem*>(A + pi_off),
+                              (uint32_t)pi.size(), 0, 0u, s, ctx));
     if (!scans.empty()) {
         MGV_CUDA_TRY(launch_cells(reinterpret_cast<ChainDev*>(A + scans_off), reinterpret_cast<BatchItem*>(A + si_off),
                                   (uint32_t)si.size(), s, ctx));
         for (const ChainDev& h : hs) MGV_CUDA_TRY(launch_cells_prefix(h.cells, s, ctx));
     }
-    MGV_CUDA_TRY(launch_batch(nullptr, reinterpret_cast<BatchOut*>(A + outs_off), nullptr, 0u,
-                              reinterpret_cast<BatchItem*>(A + ci_off), (uint32_t)ci.size(), 0, 0u, s, ctx));
+    MGV_CUDA_TRY(launch_batch_compact(reinterpret_cast<BatchOut*>(A + outs_off), reinterpret_cast<BatchItem*>(A + ci_off),
+                                      (uint32_t)ci.size(), s, ctx));
     MGV_CUDA_TRY(cudaMemcpyAsync(sl.land->counts, A + counts_off, 4ull * nq, cudaMemcpyDeviceToHost, s));
     MGV_CUDA_TRY(cudaMemcpyAsync(sl.land->rows, A + rows_off, sizeof(mgv_group_row) * std::max<uint64_t>(rows, 1),
                                  cudaMemcpyDeviceToHost, s));

@@ -112,10 +112,11 @@ mgv_status enqueue_run(mgv_batch* b, cudaStream_t s) {
     MGV_CUDA_TRY(cudaMemsetAsync(b->group_zero, 0, b->group_zero_bytes, s));
     MGV_CUDA_TRY(cudaMemsetAsync(b->out_counts, 0, sizeof(uint32_t) * b->q.size(), s));
     // every region of every table is written by the build (no clearing pass)
-    RegionJob layout{};  // the jobs themselves are on the device; this carries their slot layout
+    RegionJob layout{};  // the jobs themselves are on the device; this carries their slot layout and region size
     layout.t.key_only = b->key_only;
-    MGV_CUDA_TRY(launch_build_regions(b->d_jobs, layout, (uint32_t)b->q.size(), b->d_build_items, b->n_build, 0, 0,
-                                      b->total_regions, b->max_job_regions, b->rsc, true, false, s, ctx));
+    layout.shift = kRegionShift;
+    MGV_CUDA_TRY(launch_build_regions(b->d_jobs, layout, (uint32_t)b->q.size(), b->d_build_items, b->n_build, 0,
+                                      b->total_regions, b->max_job_regions, b->rsc, false, true, nullptr, s, ctx));
     MGV_CUDA_TRY(launch_batch(b->d_qs, b->d_probe_items, b->n_probe, (int)b->cfg.probe_ctas_per_sm, b->cfg.item_order,
                               s, ctx));
     MGV_CUDA_TRY(launch_batch_compact(b->d_outs, b->d_compact_items, b->n_compact, s, ctx));
@@ -212,17 +213,23 @@ mgv_status create_batch(mgv_ctx* ctx, const mgv_query_desc* qs, uint32_t nq, con
     for (uint32_t i = 0; i < nq; ++i) { b->out_offset[i] = out_total; out_total += qs[i].max_groups; }
     const size_t qs_off = take(sizeof(ChainDev) * std::max(nq, 1u));
     const size_t jobs_off = take(sizeof(RegionJob) * std::max(nq, 1u));
-    std::vector<uint32_t> region0(nq);
+    std::vector<uint32_t> region0(nq), share(nq);
+    std::vector<uint64_t> stage0(nq);
     uint32_t total_regions = 0, max_job_regions = 1;
-    uint64_t build_total = 0;
+    uint64_t build_total = 0, staged = 0;
     for (uint32_t i = 0; i < nq; ++i) {
         const uint32_t r = (nbk[i] + kRegionBuckets - 1) / kRegionBuckets;
         if (r > kMaxRegionsPerJob) {
             delete b;
             return fail(MGV_EUNSUPPORTED, "query " + std::to_string(i) + ": build side too large for a batch");
         }
+        TableView t{};
+        t.key_only = b->key_only;
         region0[i] = total_regions;
+        stage0[i] = staged;
+        share[i] = region_share(qs[i].build_rows, r, t, kRegionShift);
         total_regions += r;
+        staged += (uint64_t)r * share[i];
         max_job_regions = std::max(max_job_regions, r);
         build_total += qs[i].build_rows;
     }
@@ -230,7 +237,7 @@ mgv_status create_batch(mgv_ctx* ctx, const mgv_query_desc* qs, uint32_t nq, con
         delete b;
         return fail(MGV_EUNSUPPORTED, "a batch holds fewer than 2^31 build rows");
     }
-    const size_t rsc_off = take(region_scratch_bytes(total_regions, build_total));
+    const size_t rsc_off = take(region_scratch_bytes(total_regions, staged, build_total));
     const size_t outs_off = take(sizeof(BatchOut) * std::max(nq, 1u));
     b->ordered.assign(nq, 0);
     std::vector<uint32_t> sorts;
@@ -287,7 +294,7 @@ mgv_status create_batch(mgv_ctx* ctx, const mgv_query_desc* qs, uint32_t nq, con
     b->out_counts = reinterpret_cast<uint32_t*>(A + counts_off);
     b->d_qs = reinterpret_cast<ChainDev*>(A + qs_off);
     b->d_jobs = reinterpret_cast<RegionJob*>(A + jobs_off);
-    b->rsc = carve_region_scratch(A + rsc_off, total_regions, build_total);
+    b->rsc = carve_region_scratch(A + rsc_off, total_regions, staged, build_total);
     b->total_regions = total_regions;
     b->max_job_regions = max_job_regions;
     b->d_outs = reinterpret_cast<BatchOut*>(A + outs_off);
@@ -339,7 +346,7 @@ mgv_status create_batch(mgv_ctx* ctx, const mgv_query_desc* qs, uint32_t nq, con
         c.gt = g;
         c.smem_groups = std::min(gcap[i], kMaxSmemGroups);
         hj[i] = RegionJob{t, qs[i].build_keys, qs[i].build_payloads, nullptr, 0, region0[i],
-                          (nbk[i] + kRegionBuckets - 1) / kRegionBuckets, 0};
+                          (nbk[i] + kRegionBuckets - 1) / kRegionBuckets, kRegionShift, stage0[i], share[i], 0};
         // a query ordered on the device is packed there first
         mgv_group_row* packed = b->ordered[i] ? reinterpret_cast<mgv_group_row*>(A + rows_off[i])
                                               : b->h_rows_dev + b->out_offset[i];

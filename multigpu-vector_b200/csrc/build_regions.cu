@@ -3,25 +3,32 @@
 // Inserting build rows one 64-bit atomicCAS at a time into a table in global
 // memory is bound by the L2's atomic throughput (about 20 G inserts/s on
 // B200 even with the table in L2, and slower with more rows in flight).  Here
-// the table is cut into regions of kRegionBuckets buckets (64 KiB) and built
-// region by region in shared memory:
-//   1. k_region_hist     rows per region (per-CTA shared histogram per item)
-//   2. k_region_scan     exclusive prefix sum -> each region's staging range
-//   3. k_region_scatter  every row, packed {key, payload} (the key alone for a
-//                        key-only table), to its region's
-//                        range (per item: one global reservation per region,
-//                        then shared-memory cursors); for input already
-//                        partitioned on the table's radix bits,
-//                        k_region_scatter_sorted instead: each warp sorts its
-//                        256-row tile by region and stores runs
-//   4. k_region_build    one CTA per region: the region is loaded into shared
-//                        memory (or starts empty), each row claims a slot
-//                        with one shared atomicAdd on its bucket's fill
-//                        counter (linear probing on a full bucket), a
-//                        conflict-free pass finds duplicate keys, and the
-//                        region is written back with one bulk copy
-//   5. k_region_overflow rows whose run leaves their region (rare) are
-//                        inserted into the finished global table
+// the table is cut into regions of up to kRegionBuckets buckets (64 KiB) and
+// built region by region in shared memory:
+//   1. every row, packed {key, payload} (the key alone for a key-only table),
+//      goes to its region's staging range.  k_region_tile_scatter sorts tiles
+//      of thousands of rows by region in shared memory and stores runs: a lane per
+//      row to a random address is bound by the memory pipeline's request rate
+//      (4 M rows, 1024 regions: 57 us that way after a 17 us histogram and
+//      scan).  Where the ranges lie:
+//        - a table without a radix layout: the hash spreads its rows evenly,
+//          so each region has a fixed share of the staging space, twice its
+//          expected rows, and no row is counted beforehand; rows past the
+//          share join the overflow list (step 3)
+//        - a radix-laid-out table's regions follow the raw key bits, which may
+//          be skewed: exact ranges, from a histogram and a scan
+//          (k_region_hist, k_region_scan), or, for one run of a partition op
+//          with whole-region slices, inside each partition's own range
+//          (k_region_part_scatter, one CTA per partition, no global histogram)
+//   2. k_region_build    one CTA per region: each row claims a slot with one
+//                        shared atomicAdd on its bucket's fill counter (linear
+//                        probing on a full bucket), one pass finds duplicate
+//                        keys, and the region is written back with one bulk copy
+//   3. k_region_overflow rows whose run leaves their region (rare) are
+//                        inserted into the finished global table; its last CTA
+//                        hands the table's counters to the host
+// A table of one region and few rows is built by one CTA in one launch
+// (k_build_small).
 // The table is the same open-addressing table (hash_table.cuh): a row goes to
 // the first empty slot of its run from its home bucket, slots fill in order,
 // so probes are unchanged.  Rows with the reserved key INT32_MIN go to the
@@ -29,6 +36,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <type_traits>
 
 #include "device_common.cuh"
 #include "hash_table.cuh"
@@ -37,8 +45,8 @@
 namespace mgv {
 namespace {
 
-constexpr int kRBlock = 512;      // histogram / scatter CTA
-constexpr int kRBuildBlock = 512; // region build CTA
+constexpr int kRBlock = 512;       // histogram / scatter CTA
+constexpr int kRBuildBlock = 512;  // largest region build CTA: a thread per 4 buckets
 constexpr int kScanBlock = 1024;
 
 // The job of item / region lookups, cached in shared memory by the caller.
@@ -61,26 +69,69 @@ __device__ __forceinline__ BatchItem item_at(const BatchItem* items, uint32_t it
 // Staging rows: {key, payload} as 8 bytes, or the key alone (4 bytes) for a
 // key-only table -- half the scatter's stores and the build's loads.
 template <bool KO>
-__device__ __forceinline__ void stage_put(unsigned long long* staging, uint32_t pos, unsigned long long v) {
+__device__ __forceinline__ void stage_put(unsigned long long* staging, uint64_t pos, unsigned long long v) {
     if (KO) reinterpret_cast<uint32_t*>(staging)[pos] = (uint32_t)v;
     else staging[pos] = v;
 }
 
 template <bool KO>
-__device__ __forceinline__ unsigned long long stage_get(const unsigned long long* staging, uint32_t i) {
+__device__ __forceinline__ unsigned long long stage_get(const unsigned long long* staging, uint64_t i) {
     if (KO) return (unsigned long long)reinterpret_cast<const uint32_t*>(staging)[i];
     return staging[i];
 }
 
-__device__ __forceinline__ uint32_t region_of(int32_t key, const TableView& t) {
-    return home_bucket(key, t) / kRegionBuckets;
+// home_bucket (hash_table.cuh) and the region it lies in, with the table's
+// constants in registers: a job in shared memory would be read again for every
+// row, since the shared atomics between two rows could have changed it.
+struct HomeFn {
+    uint32_t radix_shift, radix_mask, bpp, shift;
+    __device__ __forceinline__ explicit HomeFn(const RegionJob& j)
+        : radix_shift(j.t.radix_shift), radix_mask(j.t.radix_mask), bpp(j.t.bpp), shift(j.shift) {}
+    __device__ __forceinline__ uint32_t bucket(int32_t key) const {
+        return (((uint32_t)key >> radix_shift) & radix_mask) * bpp + __umulhi(murmur32((uint32_t)key), bpp);
+    }
+    __device__ __forceinline__ uint32_t region(int32_t key) const { return bucket(key) >> shift; }
+};
+
+// Where a launch's rows go: staging and its region counters, and the rows
+// for the global insert.
+struct StageOut {
+    const uint32_t* start;  // exact ranges: first staging row of each region; nullptr: job.stage0 + region * job.cap
+    uint32_t* cursor;       // rows placed in each region so far
+    unsigned long long* staging;
+    unsigned long long* ovf;
+    uint32_t* ovf_job;
+    uint32_t* ctl;          // [0] rows in ovf, [1] CTAs done
+};
+
+__device__ __forceinline__ void overflow_put(const StageOut& o, unsigned long long v, uint32_t job) {
+    const uint32_t i = atomicAdd(o.ctl, 1u);
+    o.ovf[i] = v;
+    o.ovf_job[i] = job;
 }
+
+// Row `i` of a region (counted from the region's first) into its range.
+template <bool KO>
+struct StageFn {
+    const StageOut& o;
+    const uint32_t* start;
+    uint64_t stage0;
+    uint32_t cap, q;
+    __device__ __forceinline__ StageFn(const StageOut& out, const RegionJob& j, uint32_t job)
+        : o(out), start(out.start ? out.start + j.region0 : nullptr), stage0(j.stage0), cap(j.cap), q(job) {}
+    __device__ __forceinline__ void operator()(uint32_t region, uint32_t i, unsigned long long v) const {
+        if (start) stage_put<KO>(o.staging, (uint64_t)start[region] + i, v);
+        else if (i < cap) stage_put<KO>(o.staging, stage0 + (uint64_t)region * cap + i, v);
+        else overflow_put(o, v, q);
+    }
+};
 
 // Loads of kPrefetch rows per thread are issued before any is used.
 constexpr int kPrefetch = 8;
 
 // Adds the item's rows to the shared per-region counters.
 __device__ __forceinline__ void count_regions(const RegionJob& sj, const BatchItem& item, uint32_t* sh) {
+    const HomeFn home(sj);
     for (uint64_t i0 = item.lo + threadIdx.x; i0 < item.hi; i0 += (uint64_t)kRBlock * kPrefetch) {
         int32_t key[kPrefetch];
         bool in[kPrefetch];
@@ -93,11 +144,11 @@ __device__ __forceinline__ void count_regions(const RegionJob& sj, const BatchIt
         }
 #pragma unroll
         for (int u = 0; u < kPrefetch; ++u)
-            if (in[u] && key[u] != kEmptyKey) atomicAdd(sh + region_of(key[u], sj.t), 1u);
+            if (in[u] && key[u] != kEmptyKey) atomicAdd(sh + home.region(key[u]), 1u);
     }
 }
 
-__global__ void __launch_bounds__(kRBlock) k_region_hist(const RegionJob* __restrict__ jobs, RegionJob job0,
+__global__ void __launch_bounds__(kRBlock) k_region_hist(const RegionJob* __restrict__ jobs, const __grid_constant__ RegionJob job0,
                                                          const BatchItem* __restrict__ items, uint32_t nitems,
                                                          uint64_t n, uint64_t rpi, uint32_t* __restrict__ hist) {
     extern __shared__ uint32_t sh[];
@@ -120,9 +171,9 @@ __global__ void __launch_bounds__(kRBlock) k_region_hist(const RegionJob* __rest
     }
 }
 
-// One CTA: start[i] = sum of hist[0..i), start[regions] = total; cursor = start.
+// One CTA: start[i] = sum of hist[0..i), start[regions] = total.
 __global__ void __launch_bounds__(kScanBlock) k_region_scan(const uint32_t* __restrict__ hist, uint32_t regions,
-                                                            uint32_t* __restrict__ start, uint32_t* __restrict__ cursor) {
+                                                            uint32_t* __restrict__ start) {
     __shared__ uint32_t part[kScanBlock];
     const uint32_t per = (regions + kScanBlock - 1) / kScanBlock;
     const uint32_t lo = min(regions, threadIdx.x * per), hi = min(regions, lo + per);
@@ -139,17 +190,19 @@ __global__ void __launch_bounds__(kScanBlock) k_region_scan(const uint32_t* __re
     uint32_t run = part[threadIdx.x] - sum;
     for (uint32_t i = lo; i < hi; ++i) {
         start[i] = run;
-        cursor[i] = run;
         run += hist[i];
     }
     if (threadIdx.x == kScanBlock - 1) start[regions] = part[kScanBlock - 1];
 }
 
+// Rows to their regions' staging ranges one lane per row, for tables of more
+// regions than a tile sorts (kTileRegions): per item, the rows per region are
+// counted, one range per region is reserved, and shared cursors hand out its
+// rows.
 template <bool KO>
-__global__ void __launch_bounds__(kRBlock) k_region_scatter(const RegionJob* __restrict__ jobs, RegionJob job0,
+__global__ void __launch_bounds__(kRBlock) k_region_scatter(const RegionJob* __restrict__ jobs, const __grid_constant__ RegionJob job0,
                                                             const BatchItem* __restrict__ items, uint32_t nitems,
-                                                            uint64_t n, uint64_t rpi, uint32_t* __restrict__ cursor,
-                                                            unsigned long long* __restrict__ staging, uint32_t* err) {
+                                                            uint64_t n, uint64_t rpi, const __grid_constant__ StageOut out, uint32_t* err) {
     extern __shared__ uint32_t sh[];
     __shared__ RegionJob sj;
     int64_t cur = -1;
@@ -165,12 +218,14 @@ __global__ void __launch_bounds__(kRBlock) k_region_scatter(const RegionJob* __r
         __syncthreads();
         count_regions(sj, item, sh);
         __syncthreads();
-        // one reservation per region and item; sh[r] becomes the region's next staging row
+        // one reservation per region and item; sh[r] becomes the region's next row
         for (uint32_t r = threadIdx.x; r < sj.nregions; r += kRBlock) {
             const uint32_t c = sh[r];
-            if (c) sh[r] = atomicAdd(cursor + sj.region0 + r, c);
+            if (c) sh[r] = atomicAdd(out.cursor + sj.region0 + r, c);
         }
         __syncthreads();
+        const HomeFn home(sj);
+        const StageFn<KO> stage(out, sj, item.q);
         for (uint64_t i0 = item.lo + threadIdx.x; i0 < item.hi; i0 += (uint64_t)kRBlock * kPrefetch) {
             int32_t key[kPrefetch], pay[kPrefetch];
             bool in[kPrefetch];
@@ -190,130 +245,155 @@ __global__ void __launch_bounds__(kRBlock) k_region_scatter(const RegionJob* __r
                     table_insert(sj.t, key[u], pay[u], err, dup, ok);
                     continue;
                 }
-                const uint32_t pos = atomicAdd(sh + region_of(key[u], sj.t), 1u);
-                stage_put<KO>(staging, pos, ((unsigned long long)(uint32_t)pay[u] << 32) | (uint32_t)key[u]);
+                const uint32_t r = home.region(key[u]);
+                const uint32_t i = atomicAdd(sh + r, 1u);
+                stage(r, i, ((unsigned long long)(uint32_t)pay[u] << 32) | (uint32_t)key[u]);
             }
         }
     }
 }
 
-constexpr int kWarpTileRows = 8;                          // rows per lane of a warp tile
-constexpr uint32_t kWarpTile = 32u * kWarpTileRows;       // 256 rows
-constexpr uint32_t kWarpSpan = 64;                        // widest region span a warp tile sorts
+// ---- sorted tiles -------------------------------------------------------------
 
-// One warp's sorting space in k_region_scatter_sorted.
-struct WarpSort {
-    unsigned long long val[kWarpTile];  // the tile's rows in region order
-    uint32_t off[kWarpSpan];            // counts, then each region's first sorted position
-    uint32_t base[kWarpSpan];           // staging row of sorted position 0 of each region (mod 2^32)
-    uint8_t reg[kWarpTile];             // region (minus the tile's lowest) of each sorted position
+constexpr int kTileBlock = 512;
+// Rows per thread, held in registers from load to placement ({key, payload}
+// rows: 16 spill 170 bytes at 64 registers).
+template <bool KO>
+constexpr int tile_rows() { return KO ? 16 : 12; }
+template <bool KO>
+constexpr uint32_t tile_size() { return kTileBlock * tile_rows<KO>(); }
+constexpr uint32_t kTileRegions = 4096;   // most regions a tile sorts: runs of two rows on average
+constexpr uint32_t kTileCounters = 1024;  // rank counters are replicated per lane while they are at most this many
+
+// A tile's sorting space: two CTAs fit per SM up to 1024 regions.
+template <bool KO>
+struct TileSpace {
+    typename std::conditional<KO, uint32_t, unsigned long long>::type* val;  // [tile_size] rows in region order
+    uint16_t* reg;     // [tile_size] region of each sorted position
+    uint32_t* off;     // [regions * copies] counts, then first sorted positions
+    uint32_t* base;    // [regions] region row of sorted position 0 (mod 2^32)
+    uint32_t copies;   // rank counters per region: lane & (copies - 1) picks one
 };
 
-// Rows of input that is already partitioned on the table's radix bits (a
-// partition op's run: each partition's rows together, so a warp's tile of 256
-// rows falls in the regions of one or two partitions).  Each warp sorts its
-// tile by region in its own shared memory -- ranks by shared atomics, one
-// global cursor reservation per region -- and stores runs of consecutive
-// staging rows, with no block-wide barrier.  A tile whose regions span more
-// than kWarpSpan takes one cursor increment per row instead.
+__host__ __device__ constexpr uint32_t tile_copies(uint32_t regions) {
+    uint32_t f = 1;
+    while (f < 32 && 2 * f * regions <= kTileCounters) f *= 2;
+    return f;
+}
 template <bool KO>
-__global__ void __launch_bounds__(kRBlock, 2) k_region_scatter_sorted(RegionJob job, uint64_t n,
-                                                                    uint32_t* __restrict__ cursor,
-                                                                    unsigned long long* __restrict__ staging,
-                                                                    uint32_t* err) {
-    extern __shared__ __align__(16) unsigned char ws_raw[];
-    WarpSort& ws = reinterpret_cast<WarpSort*>(ws_raw)[threadIdx.x / 32];
-    const uint32_t lane = lane_id();
-    const uint64_t ntiles = (n + kWarpTile - 1) / kWarpTile;
-    const uint64_t nw = (uint64_t)gridDim.x * (kRBlock / 32);
-    for (uint64_t tile = (uint64_t)blockIdx.x * (kRBlock / 32) + threadIdx.x / 32; tile < ntiles; tile += nw) {
-        const uint64_t t0 = tile * kWarpTile;
-        int32_t key[kWarpTileRows], pay[kWarpTileRows];
-        bool in[kWarpTileRows];
+__host__ __device__ constexpr size_t tile_smem(uint32_t regions) {
+    return (KO ? 6ull : 10ull) * tile_size<KO>() + 4ull * regions * tile_copies(regions) + 4ull * regions;
+}
+template <bool KO>
+__device__ __forceinline__ TileSpace<KO> tile_space(unsigned char* base, uint32_t regions) {
+    TileSpace<KO> s;
+    s.val = reinterpret_cast<decltype(s.val)>(base);
+    s.reg = reinterpret_cast<uint16_t*>(s.val + tile_size<KO>());
+    s.copies = tile_copies(regions);
+    s.off = reinterpret_cast<uint32_t*>(s.reg + tile_size<KO>());
+    s.base = s.off + regions * s.copies;
+    return s;
+}
+
+// The rows of a tile with the reserved key, to the side list (rare: the rows
+// are read again here, so that the tile's own code keeps no insert).  Returns
+// how many were this thread's.
+__device__ __noinline__ uint32_t side_list_rows(const RegionJob& job, uint64_t lo, uint64_t hi, uint32_t* err) {
+    uint32_t rows = 0;
+    for (uint64_t i = lo + threadIdx.x; i < hi; i += kTileBlock) {
+        if (__ldg(job.keys + i) != kEmptyKey || (job.filt && __ldg(job.filt + i) > job.bound)) continue;
+        bool dup, ok;
+        table_insert(job.t, kEmptyKey, job.pays ? __ldg(job.pays + i) : 0, err, dup, ok);
+        ++rows;
+    }
+    return rows;
+}
+
+// Rows [lo, hi) (at most tile_size) of a job to their regions: ranks by shared
+// atomics, positions by a scan, one reserve(region, rows) -> first row per
+// region, then put(region, row, value) in region order, so that a warp's
+// stores are runs.  Every thread of the CTA calls it.
+template <bool KO, class Region, class Reserve, class Put>
+__device__ __forceinline__ void sort_tile(const RegionJob& job, const TileSpace<KO>& ts, uint32_t regions, uint64_t lo,
+                                          uint64_t hi, uint32_t* err, uint32_t* side_rows, Region region,
+                                          Reserve reserve, Put put) {
+    __syncthreads();  // the previous tile is stored
+    for (uint32_t r = threadIdx.x; r < regions * ts.copies; r += kTileBlock) ts.off[r] = 0;
+    const uint32_t n = (uint32_t)(hi - lo);
+    const int32_t* const keys = job.keys + lo;
+    const int32_t* const pays = !KO && job.pays ? job.pays + lo : nullptr;
+    const int32_t* const filt = job.filt ? job.filt + lo : nullptr;
+    const int32_t bound = job.bound;
+    int32_t key[tile_rows<KO>()], pay[tile_rows<KO>()];
+    uint32_t at[tile_rows<KO>()];  // region << 16 | rank, ~0 for no row
 #pragma unroll
-        for (int u = 0; u < kWarpTileRows; ++u) {
-            const uint64_t i = t0 + 32u * u + lane;
-            in[u] = i < n;
-            key[u] = in[u] ? __ldg(job.keys + i) : 0;
-            pay[u] = (in[u] && job.pays) ? __ldg(job.pays + i) : 0;
-            if (in[u] && job.filt) in[u] = __ldg(job.filt + i) <= job.bound;
-        }
-        uint32_t reg[kWarpTileRows];
-        uint32_t lo = ~0u, hi = 0;
+    for (int u = 0; u < tile_rows<KO>(); ++u) {
+        const uint32_t i = u * kTileBlock + threadIdx.x;
+        key[u] = i < n ? __ldg(keys + i) : kEmptyKey;
+        pay[u] = pays && i < n ? __ldg(pays + i) : 0;
+        at[u] = filt && i < n && __ldg(filt + i) > bound ? ~0u : 0u;
+    }
+    __syncthreads();
+    const uint32_t copy = lane_id() & (ts.copies - 1);
+    bool reserved = false;
 #pragma unroll
-        for (int u = 0; u < kWarpTileRows; ++u) {
-            reg[u] = 0;
-            if (!in[u]) continue;
-            if (key[u] == kEmptyKey) {  // the side list (its duplicates are seen from its count)
-                bool dup, ok;
-                table_insert(job.t, key[u], pay[u], err, dup, ok);
-                in[u] = false;
-                continue;
-            }
-            reg[u] = region_of(key[u], job.t);
-            lo = min(lo, reg[u]);
-            hi = max(hi, reg[u]);
-        }
-        lo = __reduce_min_sync(0xffffffffu, lo);
-        hi = __reduce_max_sync(0xffffffffu, hi);
-        if (lo > hi) continue;  // no row of the tile goes to the table
-        if (hi - lo >= kWarpSpan) {
+    for (int u = 0; u < tile_rows<KO>(); ++u) {
+        reserved |= key[u] == kEmptyKey && u * kTileBlock + threadIdx.x < n;
+        at[u] = at[u] == 0 && key[u] != kEmptyKey ? region(key[u]) << 16 : ~0u;
+    }
 #pragma unroll
-            for (int u = 0; u < kWarpTileRows; ++u)
-                if (in[u]) {
-                    const uint32_t pos = atomicAdd(cursor + job.region0 + reg[u], 1u);
-                    stage_put<KO>(staging, pos, ((unsigned long long)(uint32_t)pay[u] << 32) | (uint32_t)key[u]);
-                }
-            continue;
-        }
-        const uint32_t span = hi - lo + 1;
-        for (uint32_t j = lane; j < span; j += 32) ws.off[j] = 0;
-        __syncwarp();
-        uint32_t rank[kWarpTileRows];
+    for (int u = 0; u < tile_rows<KO>(); ++u)
+        if (at[u] != ~0u) at[u] |= atomicAdd(ts.off + (at[u] >> 16) * ts.copies + copy, 1u);
+    if (reserved) {
+        const uint32_t rows = side_list_rows(job, lo, hi, err);
+        if (side_rows && rows) atomicAdd(side_rows, rows);
+    }
+    __syncthreads();
+    const uint32_t total = block_exclusive_scan<kTileBlock>(ts.off, regions * ts.copies);
+    for (uint32_t r = threadIdx.x; r < regions; r += kTileBlock) {
+        const uint32_t first = ts.off[r * ts.copies];
+        const uint32_t c = (r + 1 < regions ? ts.off[(r + 1) * ts.copies] : total) - first;
+        ts.base[r] = (c ? reserve(r, c) : 0u) - first;
+    }
 #pragma unroll
-        for (int u = 0; u < kWarpTileRows; ++u) {
-            reg[u] -= lo;
-            rank[u] = in[u] ? atomicAdd(&ws.off[reg[u]], 1u) : 0u;
+    for (int u = 0; u < tile_rows<KO>(); ++u) {
+        if (at[u] == ~0u) continue;
+        const uint32_t r = at[u] >> 16, p = ts.off[r * ts.copies + copy] + (at[u] & 0xffffu);
+        if constexpr (KO) ts.val[p] = (uint32_t)key[u];
+        else ts.val[p] = ((unsigned long long)(uint32_t)pay[u] << 32) | (uint32_t)key[u];
+        ts.reg[p] = (uint16_t)r;
+    }
+    __syncthreads();
+#pragma unroll 4
+    for (uint32_t j = threadIdx.x; j < total; j += kTileBlock) {
+        const uint32_t r = ts.reg[j];
+        put(r, ts.base[r] + j, (unsigned long long)ts.val[j]);
+    }
+}
+
+template <bool KO>
+__global__ void __launch_bounds__(kTileBlock, 2)
+    k_region_tile_scatter(const RegionJob* __restrict__ jobs, const __grid_constant__ RegionJob job0, const BatchItem* __restrict__ items,
+                          uint32_t nitems, uint64_t n, uint64_t rpi, const __grid_constant__ StageOut out, uint32_t* err) {
+    extern __shared__ __align__(16) unsigned char tile_raw[];
+    __shared__ RegionJob sj;
+    int64_t cur = -1;
+    for (uint32_t it = blockIdx.x; it < nitems; it += gridDim.x) {
+        const BatchItem item = item_at(items, it, n, rpi);
+        if ((int64_t)item.q != cur) {
+            __syncthreads();  // the previous job's tile is stored
+            load_job(sj, jobs, job0, item.q);
+            cur = item.q;
+            __syncthreads();
         }
-        __syncwarp();
-        // lane l owns regions l and l + 32: reserve their staging ranges, then
-        // an exclusive scan of the counts gives their first sorted positions
-        const uint32_t c0 = lane < span ? ws.off[lane] : 0u;
-        const uint32_t c1 = lane + 32 < span ? ws.off[lane + 32] : 0u;
-        const uint32_t g0 = c0 ? atomicAdd(cursor + job.region0 + lo + lane, c0) : 0u;
-        const uint32_t g1 = c1 ? atomicAdd(cursor + job.region0 + lo + lane + 32, c1) : 0u;
-        uint32_t x0 = c0, x1 = c1;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t y0 = __shfl_up_sync(0xffffffffu, x0, o);
-            const uint32_t y1 = __shfl_up_sync(0xffffffffu, x1, o);
-            if (lane >= (uint32_t)o) {
-                x0 += y0;
-                x1 += y1;
-            }
-        }
-        const uint32_t tot0 = __shfl_sync(0xffffffffu, x0, 31);
-        const uint32_t total = tot0 + __shfl_sync(0xffffffffu, x1, 31);
-        const uint32_t e0 = x0 - c0, e1 = tot0 + x1 - c1;
-        if (lane < span) {
-            ws.off[lane] = e0;
-            ws.base[lane] = g0 - e0;
-        }
-        if (lane + 32 < span) {
-            ws.off[lane + 32] = e1;
-            ws.base[lane + 32] = g1 - e1;
-        }
-        __syncwarp();
-#pragma unroll
-        for (int u = 0; u < kWarpTileRows; ++u)
-            if (in[u]) {
-                const uint32_t p = ws.off[reg[u]] + rank[u];
-                ws.val[p] = ((unsigned long long)(uint32_t)pay[u] << 32) | (uint32_t)key[u];
-                ws.reg[p] = (uint8_t)reg[u];
-            }
-        __syncwarp();
-        for (uint32_t j = lane; j < total; j += 32) stage_put<KO>(staging, ws.base[ws.reg[j]] + j, ws.val[j]);
-        __syncwarp();  // the warp's buffers are free for its next tile
+        const TileSpace<KO> ts = tile_space<KO>(tile_raw, sj.nregions);
+        const HomeFn home(sj);
+        const StageFn<KO> stage(out, sj, item.q);
+        uint32_t* const cursor = out.cursor + sj.region0;
+        for (uint64_t lo = item.lo; lo < item.hi; lo += tile_size<KO>())
+            sort_tile<KO>(sj, ts, sj.nregions, lo, min(item.hi, lo + tile_size<KO>()), err, nullptr,
+                          [&](int32_t key) { return home.region(key); },
+                          [&](uint32_t r, uint32_t c) { return atomicAdd(cursor + r, c); }, stage);
     }
 }
 
@@ -365,112 +445,179 @@ __device__ __forceinline__ void bucket_keys(const unsigned long long* tab, uint3
 // has turned a row away stays full, so every row ends in the first bucket of
 // its run that had room.
 template <bool KO>
+__device__ __forceinline__ void region_put(unsigned long long* tab, uint32_t b, uint32_t q, unsigned long long v) {
+    if (KO) reinterpret_cast<uint32_t*>(tab)[8 * b + q] = (uint32_t)v;  // the key alone
+    else tab[4 * b + q] = v;
+}
+template <bool KO>
 __device__ __forceinline__ bool region_insert(unsigned long long* tab, uint32_t* fill, uint32_t nb, uint32_t b,
                                               unsigned long long v) {
     for (; b < nb; ++b) {
         const uint32_t q = atomicAdd(fill + b, 1u);
         if (q < slots_per_bucket<KO>()) {
-            if (KO) reinterpret_cast<uint32_t*>(tab)[8 * b + q] = (uint32_t)v;  // the key alone
-            else tab[4 * b + q] = v;
+            region_put<KO>(tab, b, q, v);
             return true;
         }
     }
     return false;  // the run leaves the region
 }
 
-// Whether bucket b holds a key that also appears later in its run: in b
-// itself, or in the buckets after b up to the first one that is not full.
-// Two rows with one key share their home bucket, and every bucket between
-// the two is full, so this finds every duplicate pair inside the region.
+// Whether the table region holds two rows of one key: in one bucket, or in a
+// full bucket and the buckets after it up to the first one that is not full.
+// Two rows with one key share their home bucket, and every bucket between the
+// two is full, so this finds every duplicate pair inside the region.  wrap:
+// the region is the whole table, whose runs go round its end.  A lane looks
+// into one bucket and, when it is full, walks on.  Of 8-slot buckets few are
+// full at the usual load factors (1.6 of 32 at 0.5): those are compared with
+// their successors by the whole warp, two pairs of keys a lane, instead of 64
+// pairs by one or two of its lanes (2^24 keys: 133 -> 106 us); of 4-slot
+// buckets more are (4.5 of 32), with 16 pairs each.
 template <bool KO>
-__device__ __forceinline__ bool bucket_has_dup(const unsigned long long* tab, const uint32_t* fill, uint32_t nb,
-                                               uint32_t b) {
+__device__ __forceinline__ bool region_has_dup(const unsigned long long* tab, const uint32_t* fill, uint32_t nb, bool wrap) {
     constexpr uint32_t S = slots_per_bucket<KO>();
-    const uint32_t n = min(fill[b], S);
-    if (n < 2) return false;  // no pair in b, and b is not full
-    uint32_t k[S];
-    bucket_keys<KO>(tab, b, k);
+    constexpr int kWarpWise = KO ? 4 : 0;  // full buckets of 32 that the warp takes one by one
+    const uint32_t lane = lane_id();
+    const uint32_t* words = reinterpret_cast<const uint32_t*>(tab);
     bool dup = false;
+    // the bucket `step` after f; false past the region's end
+    auto after = [&](uint32_t f, uint32_t step, uint32_t& c) {
+        c = f + step;
+        if (c < nb) return true;
+        c -= nb;
+        return wrap;
+    };
+    for (uint32_t b0 = threadIdx.x & ~31u; b0 < nb; b0 += blockDim.x) {
+        const uint32_t b = b0 + lane;
+        const uint32_t n = b < nb ? min(fill[b], S) : 0u;
+        uint32_t k[S];
+        if (n > 1) {
+            bucket_keys<KO>(tab, b, k);
 #pragma unroll
-    for (int i = 0; i < (int)S; ++i)
+            for (int j = 1; j < (int)S; ++j) {
+                bool eq = false;
 #pragma unroll
-        for (int j = i + 1; j < (int)S; ++j) dup |= (uint32_t)j < n && k[i] == k[j];
-    if (n < S) return dup;
-    for (uint32_t c = b + 1; c < nb && !dup; ++c) {
-        const uint32_t m = min(fill[c], S);
-        uint32_t o[S];
-        bucket_keys<KO>(tab, c, o);
+                for (int i = 0; i < j; ++i) eq |= k[i] == k[j];
+                dup |= eq && (uint32_t)j < n;
+            }
+        }
+        unsigned full = __ballot_sync(0xffffffffu, n == S);
+        if (__popc(full) > kWarpWise) {
+            uint32_t c;
+            for (uint32_t step = 1; n == S && !dup && step < nb && after(b, step, c); ++step) {
+                const uint32_t m = min(fill[c], S);
+                uint32_t o[S];
+                bucket_keys<KO>(tab, c, o);
 #pragma unroll
-        for (int i = 0; i < (int)S; ++i)
+                for (int j = 0; j < (int)S; ++j) {
+                    bool eq = false;
 #pragma unroll
-            for (int j = 0; j < (int)S; ++j) dup |= (uint32_t)j < m && k[i] == o[j];
-        if (m < S) break;
+                    for (int i = 0; i < (int)S; ++i) eq |= k[i] == o[j];
+                    dup |= eq && (uint32_t)j < m;
+                }
+                if (m < S) break;
+            }
+            continue;
+        }
+        for (; full; full &= full - 1) {
+            const uint32_t f = b0 + __ffs(full) - 1;
+            const uint32_t key = words[8 * f + lane / 4], j0 = lane % 4 * 2;  // against keys j0 and j0 + 1
+            uint32_t c;
+            for (uint32_t step = 1; step < nb && after(f, step, c); ++step) {
+                const uint32_t m = min(fill[c], S);
+                dup |= (j0 < m && words[8 * c + j0] == key) || (j0 + 1 < m && words[8 * c + j0 + 1] == key);
+                if (m < S) break;
+            }
+        }
     }
     return dup;
 }
 
-constexpr int kBuildRows = 8;  // staging rows per thread in one load batch (4096 per region)
+// nb empty buckets in shared memory.
+__device__ __forceinline__ void clear_table(unsigned long long* tab, uint32_t nb) {
+    const uint4 empty = make_uint4(0x80000000u, 0x80000000u, 0x80000000u, 0x80000000u);  // 2 x kEmptySlot
+    static_assert(kEmptySlot == 0x8000000080000000ull, "empty slot pattern");
+    for (uint32_t w = threadIdx.x; w < 2 * nb; w += blockDim.x) reinterpret_cast<uint4*>(tab)[w] = empty;
+}
+
+// Staging rows per thread in one load batch: at load factor 0.5 all of a region's.
+template <bool KO>
+constexpr int region_batch() { return KO ? 16 : 8; }
+
+// A region's staging rows.
+struct RegionRows {
+    uint64_t lo;
+    uint32_t n;
+};
+__device__ __forceinline__ RegionRows region_rows(const StageOut& o, const RegionJob& job, uint32_t g) {
+    if (o.start) return RegionRows{o.start[g], o.start[g + 1] - o.start[g]};
+    return RegionRows{job.stage0 + (uint64_t)(g - job.region0) * job.cap, min(o.cursor[g], job.cap)};
+}
 
 // The next region of this CTA at or after g (stride gridDim.x); without
 // `fresh`, regions that receive no rows are left as they are.
-__device__ __forceinline__ uint32_t next_region(uint32_t g, uint32_t regions, const uint32_t* start, uint32_t fresh) {
+__device__ __forceinline__ uint32_t next_region(uint32_t g, uint32_t regions, const StageOut& o, uint32_t fresh) {
     for (; g < regions; g += gridDim.x)
-        if (fresh || start[g] != start[g + 1]) return g;
+        if (fresh || (o.start ? o.start[g] != o.start[g + 1] : o.cursor[g] != 0)) return g;
     return regions;
 }
 
-// Staging rows [s0, s1) of a region, the first kBuildRows * kRBuildBlock of
-// them, into registers (rows past s1 read as empty).
-template <bool KO>
-__device__ __forceinline__ void load_region_rows(const unsigned long long* staging, uint32_t s0, uint32_t s1,
-                                                 unsigned long long (&v)[kBuildRows]) {
+// A region's rows from `from` on, one load batch, into registers (past the
+// last they read as empty).
+template <bool KO, class T>
+__device__ __forceinline__ void load_region_rows(const unsigned long long* staging, const RegionRows& rr, uint32_t from,
+                                                 T (&v)[region_batch<KO>()]) {
 #pragma unroll
-    for (int u = 0; u < kBuildRows; ++u) {
-        const uint32_t i = s0 + threadIdx.x + u * kRBuildBlock;
-        v[u] = i < s1 ? stage_get<KO>(staging, i) : kEmptySlot;
+    for (int u = 0; u < region_batch<KO>(); ++u) {
+        const uint32_t i = from + threadIdx.x + u * blockDim.x;
+        v[u] = i < rr.n ? (T)stage_get<KO>(staging, rr.lo + i) : (T)kEmptySlot;
     }
 }
 
 // Regions one at a time per CTA, several CTAs per SM; the next region's
 // first rows are loaded into registers before this region's duplicate pass
-// and bulk store, so their latency overlaps that work.
+// and bulk store, so their latency overlaps that work.  The phases of a
+// region are separated by barriers, so the SM is kept busy by its other CTAs
+// (three of 512 threads with 64 KiB regions; small tables use smaller regions
+// and CTAs, so that every SM has some).
 template <bool KO>
-__global__ void __launch_bounds__(kRBuildBlock, 3) k_region_build(const RegionJob* __restrict__ jobs, RegionJob job0,
-                                                                  uint32_t njobs, uint32_t regions,
-                                                                  const uint32_t* __restrict__ start,
-                                                                  const unsigned long long* __restrict__ staging,
-                                                                  unsigned long long* __restrict__ ovf,
-                                                                  uint32_t* ovf_count, uint32_t fresh, uint32_t* err) {
-    extern __shared__ __align__(128) unsigned long long tab[];  // kRegionBuckets * 4 slots, then the fill counters
-    uint32_t* fill = reinterpret_cast<uint32_t*>(tab + 4 * kRegionBuckets);
+__global__ void __launch_bounds__(kRBuildBlock, 3) k_region_build(const RegionJob* __restrict__ jobs, const __grid_constant__ RegionJob job0,
+                                                                  uint32_t njobs, uint32_t regions, const __grid_constant__ StageOut out,
+                                                                  uint32_t fresh, uint32_t* err) {
+    using Row = typename std::conditional<KO, uint32_t, unsigned long long>::type;
+    extern __shared__ __align__(128) unsigned long long tab[];  // the region's slots, then the fill counters
     __shared__ RegionJob sj;
     __shared__ __align__(8) uint64_t bar;
+    const uint32_t T = blockDim.x;
     if (threadIdx.x == 0) {
         mbar_init(&bar, 1);
         fence_barrier_init();
     }
     uint32_t phase = 0;
     int64_t cur = -1;
-    uint32_t g = next_region(blockIdx.x, regions, start, fresh);
-    unsigned long long v[kBuildRows];
-    if (g < regions) load_region_rows<KO>(staging, start[g], start[g + 1], v);
+    uint32_t g = next_region(blockIdx.x, regions, out, fresh);
+    uint32_t j = (jobs && njobs > 1 && g < regions) ? job_of_region(jobs, njobs, g) : 0u;
+    RegionRows rr{0, 0};
+    Row v[region_batch<KO>()];
+    if (g < regions) {
+        rr = region_rows(out, *(jobs ? jobs + j : &job0), g);
+        load_region_rows<KO>(out.staging, rr, 0, v);
+    }
     while (g < regions) {
-        const uint32_t s0 = start[g], s1 = start[g + 1];
-        const uint32_t j = (jobs && njobs > 1) ? job_of_region(jobs, njobs, g) : 0u;
         __syncthreads();  // the previous region's store has read the buffer; sj is free
         if ((int64_t)j != cur) {
             load_job(sj, jobs, job0, j);
             cur = j;
             __syncthreads();
         }
-        const uint32_t b0 = (g - sj.region0) * kRegionBuckets;
-        const uint32_t nb = min(kRegionBuckets, sj.t.nbuckets - b0);
+        const HomeFn home(sj);
+        const uint32_t rb = 1u << sj.shift;
+        const uint32_t b0 = (g - sj.region0) << sj.shift;
+        const uint32_t nb = min(rb, sj.t.nbuckets - b0);
+        uint32_t* fill = reinterpret_cast<uint32_t*>(tab + 4 * rb);
         unsigned long long* gslots = sj.t.slots + 4ull * b0;
         if (fresh) {
-            const uint4 empty = make_uint4(0x80000000u, 0x80000000u, 0x80000000u, 0x80000000u);  // 2 x kEmptySlot
-            static_assert(kEmptySlot == 0x8000000080000000ull, "empty slot pattern");
-            for (uint32_t w = threadIdx.x; w < 2 * nb; w += kRBuildBlock) reinterpret_cast<uint4*>(tab)[w] = empty;
-            for (uint32_t b = threadIdx.x; b < nb; b += kRBuildBlock) fill[b] = 0;
+            clear_table(tab, nb);
+            for (uint32_t b = threadIdx.x; b < nb; b += T) fill[b] = 0;
         } else {
             if (threadIdx.x == 0) {  // the region's current contents, one bulk copy
                 mbar_expect_tx(&bar, nb * 32);
@@ -485,7 +632,7 @@ __global__ void __launch_bounds__(kRBuildBlock, 3) k_region_build(const RegionJo
             }
             phase ^= 1u;
             // slots fill as a prefix: a bucket's count is the index of its first empty slot
-            for (uint32_t b = threadIdx.x; b < nb; b += kRBuildBlock) {
+            for (uint32_t b = threadIdx.x; b < nb; b += T) {
                 uint32_t k[slots_per_bucket<KO>()];
                 bucket_keys<KO>(tab, b, k);
                 uint32_t n = 0;
@@ -496,25 +643,27 @@ __global__ void __launch_bounds__(kRBuildBlock, 3) k_region_build(const RegionJo
         }
         __syncthreads();
         uint32_t ins = 0;
-        for (uint32_t i0 = s0 + threadIdx.x;; i0 += kRBuildBlock * kBuildRows) {
+        for (uint32_t from = 0;;) {
 #pragma unroll
-            for (int u = 0; u < kBuildRows; ++u) {
-                const uint32_t i = i0 + u * kRBuildBlock;
+            for (int u = 0; u < region_batch<KO>(); ++u) {
                 // past the region, or a gap slot of a partition's range (the
                 // reserved key goes to the side list, never into staging)
-                if (i >= s1 || (int32_t)(uint32_t)v[u] == kEmptyKey) continue;
-                const uint32_t hb = home_bucket((int32_t)(uint32_t)v[u], sj.t) - b0;
-                if (region_insert<KO>(tab, fill, nb, hb, v[u])) ++ins;
-                else ovf[atomicAdd(ovf_count, 1u)] = ((unsigned long long)j << 32) | i;  // the run leaves the region
+                if ((int32_t)(uint32_t)v[u] == kEmptyKey) continue;
+                if (region_insert<KO>(tab, fill, nb, home.bucket((int32_t)(uint32_t)v[u]) - b0, v[u])) ++ins;
+                else overflow_put(out, v[u], j);  // the run leaves the region
             }
-            if (i0 + kRBuildBlock * kBuildRows >= s1) break;
-            load_region_rows<KO>(staging, i0 + kRBuildBlock * kBuildRows - threadIdx.x, s1, v);  // a large region
+            from += T * region_batch<KO>();
+            if (from >= rr.n) break;
+            load_region_rows<KO>(out.staging, rr, from, v);  // a large region
         }
         __syncthreads();
-        const uint32_t gn = next_region(g + gridDim.x, regions, start, fresh);
-        if (gn < regions) load_region_rows<KO>(staging, start[gn], start[gn + 1], v);  // in flight from here on
-        bool dup = false;
-        for (uint32_t b = threadIdx.x; b < nb; b += kRBuildBlock) dup |= bucket_has_dup<KO>(tab, fill, nb, b);
+        const uint32_t gn = next_region(g + gridDim.x, regions, out, fresh);
+        const uint32_t jn = (jobs && njobs > 1 && gn < regions) ? job_of_region(jobs, njobs, gn) : 0u;
+        if (gn < regions) {
+            rr = region_rows(out, *(jobs ? jobs + jn : &job0), gn);
+            load_region_rows<KO>(out.staging, rr, 0, v);  // in flight from here on
+        }
+        const bool dup = region_has_dup<KO>(tab, fill, nb, false);
         fence_proxy_async_smem();  // the inserts, before the bulk store reads them
         __syncthreads();
         if (threadIdx.x == 0) {
@@ -529,25 +678,109 @@ __global__ void __launch_bounds__(kRBuildBlock, 3) k_region_build(const RegionJo
             if (any_dup) atomicOr(sj.t.meta + 3, 1ull);
         }
         g = gn;
+        j = jn;
     }
     if (threadIdx.x == 0) bulk_wait_all();  // every region store is complete before the CTA ends
 }
 
-// Rows whose run left their region, into the global table (each entry:
-// job << 32 | staging row).
-template <bool KO>
-__global__ void k_region_overflow(const RegionJob* __restrict__ jobs, RegionJob job0,
-                                  const unsigned long long* __restrict__ staging,
-                                  const unsigned long long* __restrict__ ovf, const uint32_t* ovf_count, uint32_t* err) {
-    const uint32_t cnt = *ovf_count;
+// The table's counters and the error word, to the host.
+__device__ __forceinline__ void land_table(TableLanding* land, const TableView& t, const uint32_t* err) {
+    land->err[0] = *((volatile const uint32_t*)err);
+    land->err[1] = *((volatile const uint32_t*)(err + 1));
+    for (int i = 0; i < 4; ++i) land->meta[i] = *((volatile unsigned long long*)(t.meta + i));
+}
+
+// Rows whose run left their region, into the global table; the last CTA then
+// lands the table's counters (land != nullptr: one table).
+__global__ void k_region_overflow(const RegionJob* __restrict__ jobs, const __grid_constant__ RegionJob job0, const __grid_constant__ StageOut out, TableLanding* land,
+                                  uint32_t* err) {
+    const uint32_t cnt = *out.ctl;
     for (uint32_t x = blockIdx.x * blockDim.x + threadIdx.x; x < cnt; x += gridDim.x * blockDim.x) {
-        const unsigned long long e = ovf[x];
-        const TableView t = jobs ? jobs[e >> 32].t : job0.t;
-        const unsigned long long v = stage_get<KO>(staging, (uint32_t)e);
+        const TableView t = jobs ? jobs[out.ovf_job[x]].t : job0.t;
+        const unsigned long long v = out.ovf[x];
         bool dup = false, ok = false;
         table_insert(t, (int32_t)(uint32_t)v, (int32_t)(uint32_t)(v >> 32), err, dup, ok);
         if (ok) atomicAdd(t.meta + 2, 1ull);
         if (dup) atomicOr(t.meta + 3, 1ull);
+    }
+    if (!land) return;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        if (atomicAdd(out.ctl + 1, 1u) == gridDim.x - 1) {
+            __threadfence();
+            land_table(land, job0.t, err);
+        }
+    }
+}
+
+__global__ void k_table_land(TableView t, TableLanding* land, const uint32_t* err) {
+    if (threadIdx.x == 0) land_table(land, t, err);
+}
+
+// A table of one region built from all its rows by one CTA: clear, insert,
+// duplicates, store, counters and the hand-over to the host in one launch.
+// Runs wrap around the table here, as they do in the global insert.
+constexpr int kSmallBlock = 1024;
+template <bool KO>
+__global__ void __launch_bounds__(kSmallBlock) k_build_small(const __grid_constant__ RegionJob job, uint32_t n, TableLanding* land, uint32_t* err) {
+    extern __shared__ __align__(128) unsigned long long tab[];
+    const uint32_t nb = job.t.nbuckets;
+    uint32_t* fill = reinterpret_cast<uint32_t*>(tab + 4 * nb);
+    __shared__ uint32_t s_side, s_ins, s_dup;
+    __shared__ unsigned long long s_side_sum;
+    if (threadIdx.x == 0) {
+        s_side = s_ins = s_dup = 0;
+        s_side_sum = 0;
+    }
+    clear_table(tab, nb);
+    for (uint32_t b = threadIdx.x; b < nb; b += kSmallBlock) fill[b] = 0;
+    __syncthreads();
+    uint32_t ins = 0;
+    for (uint32_t i0 = threadIdx.x; i0 < n; i0 += kSmallBlock * kPrefetch) {
+        int32_t key[kPrefetch], pay[kPrefetch];
+        bool in[kPrefetch];
+#pragma unroll
+        for (int u = 0; u < kPrefetch; ++u) {
+            const uint32_t i = i0 + u * kSmallBlock;
+            in[u] = i < n;
+            key[u] = in[u] ? __ldg(job.keys + i) : 0;
+            pay[u] = (in[u] && job.pays) ? __ldg(job.pays + i) : 0;
+            if (in[u] && job.filt) in[u] = __ldg(job.filt + i) <= job.bound;
+        }
+#pragma unroll
+        for (int u = 0; u < kPrefetch; ++u) {
+            if (!in[u]) continue;
+            if (key[u] == kEmptyKey) {
+                const uint32_t at = atomicAdd(&s_side, 1u);
+                atomicAdd(&s_side_sum, (unsigned long long)(long long)pay[u]);
+                if (at < job.t.side_cap) job.t.side_pay[at] = pay[u];
+                else set_error(err, kDevTableFull, 1);
+                continue;
+            }
+            const unsigned long long v = ((unsigned long long)(uint32_t)pay[u] << 32) | (uint32_t)key[u];
+            const uint32_t hb = home_bucket(key[u], job.t);
+            if (region_insert<KO>(tab, fill, nb, hb, v) || region_insert<KO>(tab, fill, hb, 0, v)) ++ins;
+            else set_error(err, kDevTableFull, 2);
+        }
+    }
+    __syncthreads();
+    const bool dup = region_has_dup<KO>(tab, fill, nb, true);
+    fence_proxy_async_smem();
+    ins = __reduce_add_sync(0xffffffffu, ins);
+    if (lane_id() == 0 && ins) atomicAdd(&s_ins, ins);
+    if (dup) s_dup = 1;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        bulk_s2g(job.t.slots, tab, nb * 32);
+        bulk_commit();
+        job.t.meta[0] = s_side;
+        job.t.meta[1] = s_side_sum;
+        job.t.meta[2] = s_ins;
+        job.t.meta[3] = s_dup;
+        __threadfence();
+        land_table(land, job.t, err);
+        bulk_wait_all();
     }
 }
 
@@ -562,244 +795,244 @@ __global__ void k_region_overflow(const RegionJob* __restrict__ jobs, RegionJob 
 // no global histogram, scan or cursor is needed, and the partition's rows
 // (just written by the partition op) are read from L2 twice.  Rows with the
 // reserved key go to the side list; their slots at the range's end are
-// filled with the reserved key, which the region build skips.
-constexpr int kPartScatterBlock = 1024;
-constexpr int kPartScatterRows = 8;  // loads per thread in flight
-
+// filled with the reserved key, which the region build skips.  The rows are
+// staged in sorted tiles (2^24 keys, 8 regions a partition: 89 us with a
+// match and a shared atomic per row of a warp).
 template <bool KO>
-__global__ void __launch_bounds__(kPartScatterBlock) k_region_part_scatter(RegionJob job,
-                                                                           const unsigned long long* __restrict__ ends,
-                                                                           uint32_t P, uint32_t rpp,
-                                                                           uint32_t* __restrict__ start,
-                                                                           unsigned long long* __restrict__ staging,
-                                                                           uint32_t* err) {
-    extern __shared__ uint32_t cnt[];  // rpp counters, then rpp cursors
-    uint32_t* cur = cnt + rpp;
+__global__ void __launch_bounds__(kTileBlock, 2) k_region_part_scatter(const __grid_constant__ RegionJob job,
+                                                                       const unsigned long long* __restrict__ ends,
+                                                                       uint32_t P, uint32_t rpp,
+                                                                       uint32_t* __restrict__ start,
+                                                                       unsigned long long* __restrict__ staging,
+                                                                       uint32_t* err) {
+    extern __shared__ __align__(16) unsigned char part_raw[];  // the tile space, then a row cursor per region
+    const TileSpace<KO> ts = tile_space<KO>(part_raw, rpp);
+    uint32_t* cur = ts.base + rpp;
     __shared__ uint32_t side_rows;
-    const uint32_t lane = lane_id();
-    const uint32_t bpp = job.t.bpp;
+    const uint32_t bpp = job.t.bpp, copy = lane_id() & (ts.copies - 1);
+    auto region = [&](int32_t key) { return __umulhi(murmur32((uint32_t)key), bpp) / kRegionBuckets; };
     for (uint32_t p = blockIdx.x; p < P; p += gridDim.x) {
         const uint64_t lo = p ? ends[p - 1] : 0ull, hi = ends[p];
         __syncthreads();  // the previous partition is done with the counters
-        for (uint32_t r = threadIdx.x; r < rpp; r += kPartScatterBlock) cnt[r] = 0;
+        for (uint32_t r = threadIdx.x; r < rpp * ts.copies; r += kTileBlock) ts.off[r] = 0;
         if (threadIdx.x == 0) side_rows = 0;
         __syncthreads();
         // 1. rows per region
-        for (uint64_t i0 = lo + threadIdx.x; i0 < hi; i0 += (uint64_t)kPartScatterBlock * kPartScatterRows) {
-            int32_t key[kPartScatterRows];
+        for (uint64_t i0 = lo + threadIdx.x; i0 < hi; i0 += tile_size<KO>()) {
+            int32_t key[tile_rows<KO>()];
 #pragma unroll
-            for (int u = 0; u < kPartScatterRows; ++u) {
-                const uint64_t i = i0 + (uint64_t)u * kPartScatterBlock;
+            for (int u = 0; u < tile_rows<KO>(); ++u) {
+                const uint64_t i = i0 + (uint64_t)u * kTileBlock;
                 key[u] = i < hi ? __ldg(job.keys + i) : kEmptyKey;
             }
 #pragma unroll
-            for (int u = 0; u < kPartScatterRows; ++u)
-                if (key[u] != kEmptyKey) atomicAdd(cnt + __umulhi(murmur32((uint32_t)key[u]), bpp) / kRegionBuckets, 1u);
+            for (int u = 0; u < tile_rows<KO>(); ++u)
+                if (key[u] != kEmptyKey) atomicAdd(ts.off + region(key[u]) * ts.copies + copy, 1u);
         }
         __syncthreads();
         // the regions' starts inside the partition's range
-        if (threadIdx.x < 32) {
-            uint32_t run = 0;
-            for (uint32_t r0 = 0; r0 < rpp; r0 += 32) {
-                const uint32_t r = r0 + lane;
-                const uint32_t c = r < rpp ? cnt[r] : 0u;
-                uint32_t x = c;
-#pragma unroll
-                for (int o = 1; o < 32; o <<= 1) {
-                    const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
-                    if (lane >= (uint32_t)o) x += y;
-                }
-                if (r < rpp) {
-                    const uint32_t off = (uint32_t)lo + run + x - c;
-                    cur[r] = off;
-                    start[(uint64_t)p * rpp + r] = off;
-                }
-                run += __shfl_sync(0xffffffffu, x, 31);
-            }
+        block_exclusive_scan<kTileBlock>(ts.off, rpp * ts.copies);
+        for (uint32_t r = threadIdx.x; r < rpp; r += kTileBlock) {
+            cur[r] = (uint32_t)lo + ts.off[r * ts.copies];
+            start[(uint64_t)p * rpp + r] = cur[r];
         }
         if (p == P - 1 && threadIdx.x == 0) start[(uint64_t)P * rpp] = (uint32_t)hi;
-        __syncthreads();
-        // 2. the rows, region-major; a warp's rows of one region take consecutive slots
-        for (uint64_t i0 = lo + threadIdx.x;; i0 += (uint64_t)kPartScatterBlock * kPartScatterRows) {
-            const uint64_t base = i0 - threadIdx.x;  // uniform across the CTA
-            if (base >= hi) break;
-            int32_t key[kPartScatterRows], pay[kPartScatterRows];
-#pragma unroll
-            for (int u = 0; u < kPartScatterRows; ++u) {
-                const uint64_t i = i0 + (uint64_t)u * kPartScatterBlock;
-                const bool in = i < hi;
-                key[u] = in ? __ldg(job.keys + i) : kEmptyKey;
-                pay[u] = (!KO && in && job.pays) ? __ldg(job.pays + i) : 0;
-                if (in && key[u] == kEmptyKey) {  // the side list (its duplicates are seen from its count)
-                    bool d, ok;
-                    table_insert(job.t, key[u], pay[u], err, d, ok);
-                    atomicAdd(&side_rows, 1u);
-                }
-            }
-#pragma unroll
-            for (int u = 0; u < kPartScatterRows; ++u) {
-                const bool row = key[u] != kEmptyKey;
-                const uint32_t r = row ? __umulhi(murmur32((uint32_t)key[u]), bpp) / kRegionBuckets : 0xffffffffu;
-                const uint32_t peers = __match_any_sync(0xffffffffu, r);
-                const uint32_t leader = __ffs(peers) - 1;
-                uint32_t pos = 0;
-                if (row && lane == leader) pos = atomicAdd(cur + r, (uint32_t)__popc(peers));
-                pos = __shfl_sync(0xffffffffu, pos, leader) + __popc(peers & ((1u << lane) - 1u));
-                if (row) stage_put<KO>(staging, pos, ((unsigned long long)(uint32_t)pay[u] << 32) | (uint32_t)key[u]);
-            }
-        }
+        // 2. the rows, region-major
+        for (uint64_t t0 = lo; t0 < hi; t0 += tile_size<KO>())
+            sort_tile<KO>(job, ts, rpp, t0, min(hi, t0 + tile_size<KO>()), err, &side_rows, region,
+                          [&](uint32_t r, uint32_t c) {  // one thread per region: no atomic
+                              const uint32_t at = cur[r];
+                              cur[r] = at + c;
+                              return at;
+                          },
+                          [&](uint32_t, uint32_t i, unsigned long long v) { stage_put<KO>(staging, i, v); });
         __syncthreads();
         // the reserved-key rows' slots at the end of the range
         const uint32_t nside = side_rows;
-        for (uint32_t k = threadIdx.x; k < nside; k += kPartScatterBlock)
-            stage_put<KO>(staging, (uint32_t)(hi - nside) + k, kEmptySlot);
+        for (uint32_t k = threadIdx.x; k < nside; k += kTileBlock)
+            stage_put<KO>(staging, hi - nside + k, kEmptySlot);
     }
 }
 
 }  // namespace
 
 bool region_build_partitioned_fits(const TableView& t) {
-    return t.bpp % kRegionBuckets == 0 && t.bpp / kRegionBuckets <= 4096;
+    return t.bpp % kRegionBuckets == 0 && t.bpp / kRegionBuckets <= kTileRegions;
+}
+
+static StageOut stage_out(const RegionScratch& sc, bool exact) {
+    return StageOut{exact ? sc.start : nullptr, sc.cursor, sc.staging, sc.ovf, sc.ovf_job, sc.ctl};
+}
+
+// Shared memory of k_region_build for regions of 2^shift buckets.
+static size_t region_smem(uint32_t shift) { return (32ull + 4ull) << shift; }
+
+// The region build and the global insert of what it leaves.
+static cudaError_t build_staged(const RegionJob* d_jobs, const RegionJob& job0, uint32_t njobs, uint32_t regions,
+                                uint32_t shift, const StageOut& out, bool fresh, TableLanding* land, cudaStream_t s,
+                                Context* ctx) {
+    const bool ko = job0.t.key_only != 0;
+    const void* kb = ko ? (const void*)k_region_build<true> : (const void*)k_region_build<false>;
+    const size_t smem = region_smem(shift);
+    const int block = (int)std::min((uint32_t)kRBuildBlock, (1u << shift) / 4);
+    const int grid = (int)std::min<uint64_t>(regions, (uint64_t)occupancy_grid(kb, block, smem, ctx));
+    if (ko) k_region_build<true><<<grid, block, smem, s>>>(d_jobs, job0, njobs, regions, out, fresh ? 1u : 0u, ctx->d_err);
+    else k_region_build<false><<<grid, block, smem, s>>>(d_jobs, job0, njobs, regions, out, fresh ? 1u : 0u, ctx->d_err);
+    ctx->launches++;
+    cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
+    k_region_overflow<<<ctx->prop.multiProcessorCount, 256, 0, s>>>(d_jobs, job0, out, land, ctx->d_err);
+    ctx->launches++;
+    return cudaGetLastError();
+}
+
+cudaError_t region_build_init() {
+    const size_t tab = region_smem(kRegionShift), tile_ko = tile_smem<true>(kTileRegions) + 4 * kTileRegions,
+                 tile = tile_smem<false>(kTileRegions) + 4 * kTileRegions, hist = 4ull * kMaxRegionsPerJob;
+    const struct {
+        const void* k;
+        size_t smem;
+    } all[] = {{(const void*)k_region_hist, hist},
+               {(const void*)k_region_scatter<true>, hist},
+               {(const void*)k_region_scatter<false>, hist},
+               {(const void*)k_region_tile_scatter<true>, tile_ko},
+               {(const void*)k_region_tile_scatter<false>, tile},
+               {(const void*)k_region_part_scatter<true>, tile_ko},
+               {(const void*)k_region_part_scatter<false>, tile},
+               {(const void*)k_region_build<true>, tab},
+               {(const void*)k_region_build<false>, tab},
+               {(const void*)k_build_small<true>, tab},
+               {(const void*)k_build_small<false>, tab}};
+    for (const auto& x : all) {
+        const cudaError_t e = cudaFuncSetAttribute(x.k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)x.smem);
+        if (e != cudaSuccess) return e;
+    }
+    return cudaSuccess;
 }
 
 cudaError_t launch_build_regions_partitioned(const RegionJob& job, const unsigned long long* ends, uint64_t n,
-                                             const RegionScratch& sc, cudaStream_t s, Context* ctx) {
+                                             const RegionScratch& sc, TableLanding* land, cudaStream_t s, Context* ctx) {
     const uint32_t P = job.t.radix_mask + 1;
     const uint32_t rpp = job.t.bpp / kRegionBuckets;
     const uint32_t regions = P * rpp;
     const bool ko = job.t.key_only != 0;
-    const size_t psmem = 8ull * rpp;
-    const size_t tsmem = (32ull + 4ull) * kRegionBuckets;
-    const void* kp = ko ? (const void*)k_region_part_scatter<true> : (const void*)k_region_part_scatter<false>;
-    const void* kb = ko ? (const void*)k_region_build<true> : (const void*)k_region_build<false>;
     cudaError_t e;
-    if ((e = cudaFuncSetAttribute(kp, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)psmem)) ||
-        (e = cudaFuncSetAttribute(kb, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tsmem)))
-        return e;
-    if ((e = cudaMemsetAsync(sc.ovf_count, 0, 4, s))) return e;
+    if ((e = cudaMemsetAsync(sc.cursor, 0, region_zero_bytes(regions), s))) return e;
     if (n) {
-        const int grid = (int)std::min<uint64_t>(P, (uint64_t)occupancy_grid(kp, kPartScatterBlock, psmem, ctx));
+        const size_t smem = (ko ? tile_smem<true>(rpp) : tile_smem<false>(rpp)) + 4ull * rpp;
+        const void* kp = ko ? (const void*)k_region_part_scatter<true> : (const void*)k_region_part_scatter<false>;
+        const int grid = (int)std::min<uint64_t>(P, (uint64_t)occupancy_grid(kp, kTileBlock, smem, ctx));
         if (ko)
-            k_region_part_scatter<true><<<grid, kPartScatterBlock, psmem, s>>>(job, ends, P, rpp, sc.start, sc.staging,
-                                                                                ctx->d_err);
+            k_region_part_scatter<true><<<grid, kTileBlock, smem, s>>>(job, ends, P, rpp, sc.start, sc.staging, ctx->d_err);
         else
-            k_region_part_scatter<false><<<grid, kPartScatterBlock, psmem, s>>>(job, ends, P, rpp, sc.start,
-                                                                                 sc.staging, ctx->d_err);
+            k_region_part_scatter<false><<<grid, kTileBlock, smem, s>>>(job, ends, P, rpp, sc.start, sc.staging, ctx->d_err);
         ctx->launches++;
         if ((e = cudaGetLastError())) return e;
     } else {  // nothing staged: every region is empty
         if ((e = cudaMemsetAsync(sc.start, 0, 4ull * (regions + 1), s))) return e;
     }
-    const int grid = (int)std::min<uint64_t>(regions, (uint64_t)occupancy_grid(kb, kRBuildBlock, tsmem, ctx));
-    if (ko)
-        k_region_build<true><<<grid, kRBuildBlock, tsmem, s>>>(nullptr, job, 1, regions, sc.start, sc.staging, sc.ovf,
-                                                               sc.ovf_count, 1u, ctx->d_err);
-    else
-        k_region_build<false><<<grid, kRBuildBlock, tsmem, s>>>(nullptr, job, 1, regions, sc.start, sc.staging,
-                                                                sc.ovf, sc.ovf_count, 1u, ctx->d_err);
-    ctx->launches++;
-    if ((e = cudaGetLastError())) return e;
-    const int sms = ctx->prop.multiProcessorCount;
-    if (ko) k_region_overflow<true><<<sms * 2, 256, 0, s>>>(nullptr, job, sc.staging, sc.ovf, sc.ovf_count, ctx->d_err);
-    else k_region_overflow<false><<<sms * 2, 256, 0, s>>>(nullptr, job, sc.staging, sc.ovf, sc.ovf_count, ctx->d_err);
-    ctx->launches++;
-    return cudaGetLastError();
+    return build_staged(nullptr, job, 1, regions, kRegionShift, stage_out(sc, true), true, land, s, ctx);
 }
 
-size_t region_scratch_bytes(uint32_t regions, uint64_t rows) {
-    auto a = [](size_t x) { return (x + 255) & ~(size_t)255; };
-    return a(4ull * regions) + a(4ull * (regions + 1)) + a(4ull * regions) + a(4) + a(8ull * rows) + a(8ull * rows);
+static size_t align_scratch(size_t x) { return (x + 255) & ~(size_t)255; }
+
+size_t region_zero_bytes(uint32_t regions) { return align_scratch(4ull * regions) + 8; }
+
+size_t region_scratch_bytes(uint32_t regions, uint64_t staged, uint64_t rows) {
+    auto a = align_scratch;
+    return a(region_zero_bytes(regions)) + a(4ull * regions) + a(4ull * (regions + 1)) + a(8ull * staged) + a(8ull * rows) +
+           a(4ull * rows);
 }
 
-RegionScratch carve_region_scratch(void* base, uint32_t regions, uint64_t rows) {
-    auto a = [](size_t x) { return (x + 255) & ~(size_t)255; };
+RegionScratch carve_region_scratch(void* base, uint32_t regions, uint64_t staged, uint64_t rows) {
+    auto a = align_scratch;
     unsigned char* p = static_cast<unsigned char*>(base);
     RegionScratch s;
+    s.cursor = reinterpret_cast<uint32_t*>(p);
+    s.ctl = reinterpret_cast<uint32_t*>(p + a(4ull * regions));
+    p += a(region_zero_bytes(regions));
     s.hist = reinterpret_cast<uint32_t*>(p);
     p += a(4ull * regions);
     s.start = reinterpret_cast<uint32_t*>(p);
     p += a(4ull * (regions + 1));
-    s.cursor = reinterpret_cast<uint32_t*>(p);
-    p += a(4ull * regions);
-    s.ovf_count = reinterpret_cast<uint32_t*>(p);
-    p += a(4);
     s.staging = reinterpret_cast<unsigned long long*>(p);
-    p += a(8ull * rows);
+    p += a(8ull * staged);
     s.ovf = reinterpret_cast<unsigned long long*>(p);
+    p += a(8ull * rows);
+    s.ovf_job = reinterpret_cast<uint32_t*>(p);
     return s;
 }
 
+uint32_t region_share(uint64_t rows, uint32_t nregions, const TableView& t, uint32_t shift) {
+    const uint64_t slots = (uint64_t)(t.key_only ? 8 : 4) << shift;
+    const uint64_t expected = (rows + nregions - 1) / nregions;
+    return (uint32_t)std::max<uint64_t>(1, std::min({slots, 2 * expected + 256, rows}));
+}
+
 cudaError_t launch_build_regions(const RegionJob* d_jobs, const RegionJob& job0, uint32_t njobs,
-                                 const BatchItem* items, uint32_t nitems, uint64_t n, uint64_t rows_per_item,
-                                 uint32_t total_regions, uint32_t max_job_regions, const RegionScratch& sc,
-                                 bool fresh, bool partitioned, cudaStream_t s, Context* ctx) {
+                                 const BatchItem* items, uint32_t nitems, uint64_t n, uint32_t total_regions,
+                                 uint32_t max_job_regions, const RegionScratch& sc, bool exact, bool fresh,
+                                 TableLanding* land, cudaStream_t s, Context* ctx) {
     if (total_regions == 0) return cudaSuccess;
-    if (!items) nitems = (uint32_t)((n + rows_per_item - 1) / rows_per_item);
-    const int sms = ctx->prop.multiProcessorCount;
-    const size_t hsmem = 4ull * std::max(max_job_regions, 1u);
-    const bool sorted = partitioned && !items && njobs == 1;
-    const size_t wsmem = sizeof(WarpSort) * (kRBlock / 32);
-    const size_t tsmem = (32ull + 4ull) * kRegionBuckets;  // the region, then its fill counters
     // every job of one launch has the same slot layout (all key-only or none); a
     // key-only launch stages 4-byte keys
     const bool ko = job0.t.key_only != 0;
-    const void* kscat = ko ? (const void*)k_region_scatter<true> : (const void*)k_region_scatter<false>;
-    const void* ksort = ko ? (const void*)k_region_scatter_sorted<true> : (const void*)k_region_scatter_sorted<false>;
+    const bool tiles = max_job_regions <= kTileRegions;
+    const size_t hsmem = 4ull * std::max(max_job_regions, 1u);
+    const size_t smem = !tiles ? hsmem : ko ? tile_smem<true>(max_job_regions) : tile_smem<false>(max_job_regions);
+    const void* k = tiles ? (ko ? (const void*)k_region_tile_scatter<true> : (const void*)k_region_tile_scatter<false>)
+                          : (ko ? (const void*)k_region_scatter<true> : (const void*)k_region_scatter<false>);
+    const uint64_t ctas = (uint64_t)occupancy_grid(k, tiles ? kTileBlock : kRBlock, smem, ctx);
+    const uint64_t tile = ko ? tile_size<true>() : tile_size<false>();
+    uint64_t rpi = 0;
+    if (!items && n) {
+        // whole tiles dealt evenly over the CTAs, or items worth zeroing and flushing their region counters
+        if (tiles) rpi = (n - 1) / (ctas * ((n - 1) / (ctas * tile) + 1)) + 1;
+        else rpi = std::max<uint64_t>({8ull * max_job_regions, 4096, n / (2ull * ctx->prop.multiProcessorCount) + 1});
+        nitems = (uint32_t)((n + rpi - 1) / rpi);
+    }
     cudaError_t e;
-    if ((e = cudaFuncSetAttribute(k_region_hist, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)hsmem)) ||
-        (e = cudaFuncSetAttribute(kscat, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)hsmem)) ||
-        (e = cudaFuncSetAttribute(ksort, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)wsmem)) ||
-        (e = cudaFuncSetAttribute(k_region_build<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tsmem)) ||
-        (e = cudaFuncSetAttribute(k_region_build<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tsmem)))
-        return e;
-    if ((e = cudaMemsetAsync(sc.hist, 0, 4ull * total_regions, s))) return e;
-    if ((e = cudaMemsetAsync(sc.ovf_count, 0, 4, s))) return e;
+    if ((e = cudaMemsetAsync(sc.cursor, 0, region_zero_bytes(total_regions), s))) return e;
+    if (exact) {
+        if ((e = cudaMemsetAsync(sc.hist, 0, 4ull * total_regions, s))) return e;
+        if (nitems) {
+            const int grid = (int)std::min<uint64_t>(nitems, (uint64_t)occupancy_grid((const void*)k_region_hist, kRBlock,
+                                                                                       hsmem, ctx));
+            k_region_hist<<<grid, kRBlock, hsmem, s>>>(d_jobs, job0, items, nitems, n, rpi, sc.hist);
+            ctx->launches++;
+            if ((e = cudaGetLastError())) return e;
+        }
+        k_region_scan<<<1, kScanBlock, 0, s>>>(sc.hist, total_regions, sc.start);
+        ctx->launches++;
+        if ((e = cudaGetLastError())) return e;
+    }
+    const StageOut out = stage_out(sc, exact);
     if (nitems) {
-        const int grid = (int)std::min<uint64_t>(nitems, (uint64_t)occupancy_grid((const void*)k_region_hist, kRBlock,
-                                                                                   hsmem, ctx));
-        k_region_hist<<<grid, kRBlock, hsmem, s>>>(d_jobs, job0, items, nitems, n, rows_per_item, sc.hist);
+        const int grid = (int)std::min<uint64_t>(nitems, ctas);
+        if (tiles && ko)
+            k_region_tile_scatter<true><<<grid, kTileBlock, smem, s>>>(d_jobs, job0, items, nitems, n, rpi, out, ctx->d_err);
+        else if (tiles)
+            k_region_tile_scatter<false><<<grid, kTileBlock, smem, s>>>(d_jobs, job0, items, nitems, n, rpi, out, ctx->d_err);
+        else if (ko)
+            k_region_scatter<true><<<grid, kRBlock, smem, s>>>(d_jobs, job0, items, nitems, n, rpi, out, ctx->d_err);
+        else
+            k_region_scatter<false><<<grid, kRBlock, smem, s>>>(d_jobs, job0, items, nitems, n, rpi, out, ctx->d_err);
         ctx->launches++;
         if ((e = cudaGetLastError())) return e;
     }
-    k_region_scan<<<1, kScanBlock, 0, s>>>(sc.hist, total_regions, sc.start, sc.cursor);
+    return build_staged(d_jobs, job0, njobs, total_regions, job0.shift, out, fresh, land, s, ctx);
+}
+
+cudaError_t launch_build_small(const RegionJob& job, uint32_t n, TableLanding* land, cudaStream_t s, Context* ctx) {
+    const size_t smem = 36ull * job.t.nbuckets;
+    if (job.t.key_only) k_build_small<true><<<1, kSmallBlock, smem, s>>>(job, n, land, ctx->d_err);
+    else k_build_small<false><<<1, kSmallBlock, smem, s>>>(job, n, land, ctx->d_err);
     ctx->launches++;
-    if ((e = cudaGetLastError())) return e;
-    if (sorted && n) {
-        const uint64_t tiles = (n + kWarpTile - 1) / kWarpTile;
-        const uint64_t ctas = (tiles + kRBlock / 32 - 1) / (kRBlock / 32);
-        const int grid = (int)std::min<uint64_t>(ctas, (uint64_t)occupancy_grid(ksort, kRBlock, wsmem, ctx));
-        if (ko) k_region_scatter_sorted<true><<<grid, kRBlock, wsmem, s>>>(job0, n, sc.cursor, sc.staging, ctx->d_err);
-        else k_region_scatter_sorted<false><<<grid, kRBlock, wsmem, s>>>(job0, n, sc.cursor, sc.staging, ctx->d_err);
-        ctx->launches++;
-        if ((e = cudaGetLastError())) return e;
-    } else if (nitems) {
-        const int grid = (int)std::min<uint64_t>(nitems, (uint64_t)occupancy_grid(kscat, kRBlock, hsmem, ctx));
-        if (ko)
-            k_region_scatter<true><<<grid, kRBlock, hsmem, s>>>(d_jobs, job0, items, nitems, n, rows_per_item,
-                                                                sc.cursor, sc.staging, ctx->d_err);
-        else
-            k_region_scatter<false><<<grid, kRBlock, hsmem, s>>>(d_jobs, job0, items, nitems, n, rows_per_item,
-                                                                 sc.cursor, sc.staging, ctx->d_err);
-        ctx->launches++;
-        if ((e = cudaGetLastError())) return e;
-    }
-    {
-        const void* kb = ko ? (const void*)k_region_build<true> : (const void*)k_region_build<false>;
-        const int grid = (int)std::min<uint64_t>(total_regions,
-                                                 (uint64_t)occupancy_grid(kb, kRBuildBlock, tsmem, ctx));
-        if (ko)
-            k_region_build<true><<<grid, kRBuildBlock, tsmem, s>>>(d_jobs, job0, njobs, total_regions, sc.start,
-                                                                   sc.staging, sc.ovf, sc.ovf_count, fresh ? 1u : 0u,
-                                                                   ctx->d_err);
-        else
-            k_region_build<false><<<grid, kRBuildBlock, tsmem, s>>>(d_jobs, job0, njobs, total_regions, sc.start,
-                                                                    sc.staging, sc.ovf, sc.ovf_count,
-                                                                    fresh ? 1u : 0u, ctx->d_err);
-        ctx->launches++;
-        if ((e = cudaGetLastError())) return e;
-    }
-    if (ko) k_region_overflow<true><<<sms * 2, 256, 0, s>>>(d_jobs, job0, sc.staging, sc.ovf, sc.ovf_count, ctx->d_err);
-    else k_region_overflow<false><<<sms * 2, 256, 0, s>>>(d_jobs, job0, sc.staging, sc.ovf, sc.ovf_count, ctx->d_err);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_table_land(const TableView& t, TableLanding* land, cudaStream_t s, Context* ctx) {
+    k_table_land<<<1, 32, 0, s>>>(t, land, ctx->d_err);
     ctx->launches++;
     return cudaGetLastError();
 }

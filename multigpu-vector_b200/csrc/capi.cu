@@ -226,6 +226,7 @@ mgv_status mgv_ctx_create(int device, mgv_ctx** out) {
     if (e == cudaSuccess) e = cudaMemset(c->d_err, 0, 2 * sizeof(uint32_t));
     if (e == cudaSuccess) e = cudaMallocHost(&c->h_stage, 8 * sizeof(unsigned long long));
     if (e == cudaSuccess) e = group_rows_init();
+    if (e == cudaSuccess) e = region_build_init();
     if (e != cudaSuccess) {
         if (c->h_stage) cudaFreeHost(c->h_stage);
         if (c->d_err) cudaFree(c->d_err);
@@ -561,8 +562,14 @@ mgv_status mgv_op_create_hash_build(mgv_ctx* ctx, const mgv_hash_build_desc* d, 
     mgv_status st = dev_alloc(o, (void**)&t.slots, o->table_bytes);
     if (st == MGV_OK) st = dev_alloc(o, (void**)&t.meta, 4 * sizeof(unsigned long long));
     if (st == MGV_OK) st = dev_alloc(o, (void**)&t.side_pay, sizeof(int32_t) * t.side_cap);
-    if (st == MGV_OK && cudaMallocHost(&o->h_res, 5 * sizeof(unsigned long long)) != cudaSuccess)
-        st = fail(MGV_ENOMEM, "pinned host allocation");
+    if (st == MGV_OK) {
+        cudaError_t e = cudaMallocHost(&o->hb_land, sizeof(TableLanding));
+        if (e == cudaSuccess) e = cudaHostGetDevicePointer(reinterpret_cast<void**>(&o->hb_land_dev), o->hb_land, 0);
+        if (e != cudaSuccess) {
+            if (o->hb_land) cudaFreeHost(o->hb_land);
+            st = fail(MGV_ENOMEM, "pinned host allocation");
+        }
+    }
     if (st != MGV_OK) {
         for (void* p : o->allocs) cudaFree(p);
         delete o;
@@ -711,6 +718,7 @@ mgv_status mgv_op_destroy(mgv_op* o) {
     for (cudaEvent_t ev : o->in_consumed)
         if (ev) cudaEventDestroy(ev);
     if (o->h_res) cudaFreeHost(o->h_res);
+    if (o->hb_land) cudaFreeHost(o->hb_land);
     if (o->rb_scratch) cudaFree(o->rb_scratch);
     if (o->gb_land) cudaFreeHost(o->gb_land);
     for (void* p : o->allocs) cudaFree(p);
@@ -726,10 +734,11 @@ static mgv_status op_reset(Op* o, cudaStream_t s) {
             o->agg_result = mgv_agg_result{0, 0};
             break;
         case OpKind::HashBuild:
-            // The table is cleared lazily: a first shared-memory build writes
-            // every bucket itself; otherwise the first consume (or close) fills it.
-            MGV_CUDA_TRY(cudaMemsetAsync(o->table.meta, 0, 4 * sizeof(unsigned long long), s));
+            // The table and its counters are cleared lazily: a first shared-memory
+            // build writes every bucket itself; otherwise the first consume (or
+            // close) fills them.
             o->hb_fresh = true;
+            o->hb_landed = false;
             o->unique = false;
             break;
         case OpKind::Sink: {
@@ -834,6 +843,7 @@ mgv_status mgv_op_close(mgv_op* o, void* stream) {
         if (st != MGV_OK) return st;
     }
     if (o->kind == OpKind::HashBuild && o->hb_fresh) {  // nothing was built: clear the table now
+        MGV_CUDA_TRY(cudaMemsetAsync(o->table.meta, 0, 4 * sizeof(unsigned long long), s));
         MGV_CUDA_TRY(launch_fill_u64(o->table.slots, 4ull * o->table.nbuckets, kEmptySlot, s, o->ctx));
         o->hb_fresh = false;
     }
@@ -850,15 +860,12 @@ mgv_status mgv_op_close(mgv_op* o, void* stream) {
             return report_device_error(o->ctx, w, s);
         }
         if (o->kind == OpKind::Groupby) return close_groupby(o, s);
-        if (o->kind == OpKind::HashBuild) {  // the error word and the table's counters: one copy, one wait
-            unsigned long long* h = o->h_res;
-            MGV_CUDA_TRY(cudaMemcpyAsync(h, o->ctx->d_err, 2 * sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
-            MGV_CUDA_TRY(cudaMemcpyAsync(h + 1, o->table.meta, 4 * sizeof(unsigned long long), cudaMemcpyDeviceToHost,
-                                         s));
+        if (o->kind == OpKind::HashBuild) {  // the error word and the table's counters, with one wait
+            if (!o->hb_landed) MGV_CUDA_TRY(launch_table_land(o->table, o->hb_land_dev, s, o->ctx));
             MGV_CUDA_TRY(cudaStreamSynchronize(s));
-            const uint32_t w[2] = {reinterpret_cast<uint32_t*>(h)[0], reinterpret_cast<uint32_t*>(h)[1]};
+            const uint32_t w[2] = {o->hb_land->err[0], o->hb_land->err[1]};
             st = report_device_error(o->ctx, w, s);
-            if (st == MGV_OK) hash_build_info(o, h + 1);
+            if (st == MGV_OK) hash_build_info(o, o->hb_land->meta);
             return st;
         }
         st = check_device(o->ctx, s);
@@ -892,15 +899,14 @@ mgv_status mgv_op_close(mgv_op* o, void* stream) {
         }
         if (st == MGV_OK && o->pt_fill) {
             Op* hb = o->parent;
-            hb->hb_partitioned = hb->kind == OpKind::HashBuild && hb->hb.key_col == o->pt.key_col &&
-                                 hb->table.radix_mask == (1u << o->pt.radix_bits) - 1u &&
-                                 hb->table.radix_shift == o->pt.radix_shift;
+            const bool same_bits = hb->kind == OpKind::HashBuild && hb->hb.key_col == o->pt.key_col &&
+                                   hb->table.radix_mask == (1u << o->pt.radix_bits) - 1u &&
+                                   hb->table.radix_shift == o->pt.radix_shift;
             // one run: the partition ends left by its scatter locate each partition's rows
-            hb->hb_part_ends = hb->hb_partitioned && o->pt_runs == 1 ? o->pt_dev : nullptr;
+            hb->hb_part_ends = same_bits && o->pt_runs == 1 ? o->pt_dev : nullptr;
             const int32_t* cols[MGV_MAX_COLS];
             for (uint32_t c = 0; c < o->pt_ncols; ++c) cols[c] = o->pt_store + c * o->pt.max_rows;
             st = consume_cols(o->parent, cols, o->pt_ncols, o->pt_fill, s);
-            hb->hb_partitioned = false;
             hb->hb_part_ends = nullptr;
         }
     }
@@ -1161,17 +1167,38 @@ static mgv_status consume_cols(Op* head, const int32_t* const* cols, uint32_t nc
             const int32_t* pays = pc >= 0 ? cols[pc] : nullptr;
             const int32_t* filt = sel ? cols[sel->sel.col] : nullptr;
             const int32_t bound = sel ? sel->sel.bound : 0;
-            const uint32_t regions = table_regions(term->table);
+            const TableView& t = term->table;
             const bool fresh = term->hb_fresh;
             term->hb_fresh = false;
-            if (n < kRegionBuildMinRows || n >= (1ull << 31) || regions > kMaxRegionsPerJob) {
-                if (fresh)
-                    MGV_CUDA_TRY(launch_fill_u64(term->table.slots, 4ull * term->table.nbuckets, kEmptySlot, s, ctx));
-                MGV_CUDA_TRY(launch_build(cols[kc], pays, filt, bound, sel != nullptr, n, term->table, s, ctx));
+            term->hb_landed = false;
+            RegionJob job{t, cols[kc], pays, filt, bound, 0, 1, kRegionShift, 0, 0, 0};
+            // a table of one region and few rows: one CTA reads them in a few
+            // microseconds, less than a second launch costs
+            if (fresh && t.nbuckets <= kRegionBuckets && n <= kSmallBuildRows) {
+                MGV_CUDA_TRY(launch_build_small(job, (uint32_t)n, term->hb_land_dev, s, ctx));
+                term->hb_landed = true;
                 return MGV_OK;
             }
-            // shared-memory build; its scratch is kept by the operator and grown on demand
-            const size_t need = region_scratch_bytes(regions, n);
+            if (fresh) MGV_CUDA_TRY(cudaMemsetAsync(t.meta, 0, 4 * sizeof(unsigned long long), s));
+            if (n < kRegionBuildMinRows || n >= (1ull << 31) || table_regions(t) > kMaxRegionsPerJob) {
+                if (fresh) MGV_CUDA_TRY(launch_fill_u64(t.slots, 4ull * t.nbuckets, kEmptySlot, s, ctx));
+                MGV_CUDA_TRY(launch_build(cols[kc], pays, filt, bound, sel != nullptr, n, t, s, ctx));
+                return MGV_OK;
+            }
+            // the hash spreads an unpartitioned table's rows evenly: fixed staging shares,
+            // and regions small enough for two per SM; a radix layout follows the raw
+            // key bits: exact staging ranges
+            const bool exact = t.radix_mask != 0;
+            const bool part_run = fresh && term->hb_part_ends && !sel && region_build_partitioned_fits(t);
+            if (!exact)
+                while (job.shift > kMinRegionShift &&
+                       (t.nbuckets >> job.shift) < 2u * (uint32_t)ctx->prop.multiProcessorCount)
+                    --job.shift;
+            job.nregions = (t.nbuckets + (1u << job.shift) - 1) >> job.shift;
+            job.cap = region_share(n, job.nregions, t, job.shift);
+            const uint64_t staged = exact ? n : (uint64_t)job.nregions * job.cap;
+            // the scratch is kept by the operator and grown on demand
+            const size_t need = region_scratch_bytes(job.nregions, staged, n);
             if (term->rb_bytes < need) {
                 if (term->rb_scratch) {
                     MGV_CUDA_TRY(cudaStreamSynchronize(s));
@@ -1182,19 +1209,13 @@ static mgv_status consume_cols(Op* head, const int32_t* const* cols, uint32_t nc
                 MGV_CUDA_TRY(cudaMalloc(&term->rb_scratch, need));
                 term->rb_bytes = need;
             }
-            const RegionJob job{term->table, cols[kc], pays, filt, bound, 0, regions, 0};
-            if (fresh && term->hb_part_ends && !sel && region_build_partitioned_fits(term->table)) {
-                MGV_CUDA_TRY(launch_build_regions_partitioned(job, term->hb_part_ends, n,
-                                                              carve_region_scratch(term->rb_scratch, regions, n), s,
-                                                              ctx));
-                return MGV_OK;
-            }
-            // items: two per SM, each worth zeroing and flushing its region histogram
-            const uint64_t rows_per_item =
-                std::max<uint64_t>({8ull * regions, 4096, n / (2ull * ctx->prop.multiProcessorCount) + 1});
-            MGV_CUDA_TRY(launch_build_regions(nullptr, job, 1, nullptr, 0, n, rows_per_item, regions, regions,
-                                              carve_region_scratch(term->rb_scratch, regions, n), fresh,
-                                              term->hb_partitioned && !sel, s, ctx));
+            const RegionScratch sc = carve_region_scratch(term->rb_scratch, job.nregions, staged, n);
+            if (part_run)
+                MGV_CUDA_TRY(launch_build_regions_partitioned(job, term->hb_part_ends, n, sc, term->hb_land_dev, s, ctx));
+            else
+                MGV_CUDA_TRY(launch_build_regions(nullptr, job, 1, nullptr, 0, n, job.nregions, job.nregions, sc, exact,
+                                                  fresh, term->hb_land_dev, s, ctx));
+            term->hb_landed = true;
             return MGV_OK;
         }
         case OpKind::Partition: {

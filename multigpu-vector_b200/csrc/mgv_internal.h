@@ -188,8 +188,10 @@ struct Op {
     unsigned long long* pt_dev = nullptr; // [P] histogram / cursors of a consume
     unsigned long long* pt_acc = nullptr; // [1 + P] rows stored, rows per partition
     std::vector<uint64_t> pt_hist;        // rows per partition (read back at close)
-    bool hb_fresh = false;  // opened, nothing consumed yet: the table is not cleared yet
-    bool hb_partitioned = false;  // the rows being consumed are a partition op's run on the table's radix bits
+    bool hb_fresh = false;  // opened, nothing consumed yet: the table and its counters are not cleared yet
+    bool hb_landed = false;  // the last consume's kernels hand the table's counters to the host
+    struct TableLanding* hb_land = nullptr;  // pinned, mapped
+    struct TableLanding* hb_land_dev = nullptr;
     const unsigned long long* hb_part_ends = nullptr;  // that run's partition ends (device), when it is the only run
     // host ingest (mgv_op_consume_host): the copy stream and, per buffer in
     // flight, events for "slice copied" and "slice consumed"
@@ -327,9 +329,15 @@ struct BatchItem {  // rows [lo, hi) of query q
 // a shared-memory copy of the region and writes it back with coalesced
 // stores.  A row whose run leaves its region is inserted afterwards into the
 // global table.  A "job" is one table's build; a launch can build many.
-constexpr uint32_t kRegionBuckets = 2048;      // 64 KiB of table per region
+constexpr uint32_t kRegionShift = 11;
+constexpr uint32_t kRegionBuckets = 1u << kRegionShift;  // 64 KiB of table per region
+// Small tables: smaller regions, so that every SM gets some.  300 K {key,
+// payload} rows, regions of 2^11 / 2^10 / 2^9 / 2^8 buckets: staging, build and
+// global insert take 54 / 53 / 61 / 62 us (every region end adds rows to the insert).
+constexpr uint32_t kMinRegionShift = 10;
 constexpr uint32_t kMaxRegionsPerJob = 16384;  // per-CTA region histogram: 64 KiB
 constexpr uint64_t kRegionBuildMinRows = 1u << 16;  // smaller builds: one global CAS per row
+constexpr uint64_t kSmallBuildRows = 1u << 14;      // a one-region table of at most this many rows: one CTA, one launch
 struct RegionJob {
     TableView t;
     const int32_t* keys;
@@ -337,38 +345,54 @@ struct RegionJob {
     const int32_t* filt;      // nullable: rows with filt <= bound only
     int32_t bound;
     uint32_t region0;         // first region of this job in the launch
-    uint32_t nregions;
+    uint32_t nregions;        // regions of 2^shift buckets
+    uint32_t shift;
+    uint64_t stage0;          // region r's staging rows: stage0 + r * cap on (when the ranges are not exact)
+    uint32_t cap;
     uint32_t pad;
 };
 struct RegionScratch {
-    uint32_t* hist;           // [regions] rows per region
-    uint32_t* start;          // [regions + 1] first staging row of each region
-    uint32_t* cursor;         // [regions]
-    uint32_t* ovf_count;      // [1]
-    unsigned long long* staging;  // [rows] {key, payload}, region-major
-    unsigned long long* ovf;  // [rows] job << 32 | staging row, left for the global insert
+    uint32_t* cursor;         // [regions] rows placed, zeroed together with ctl (region_zero_bytes)
+    uint32_t* ctl;            // [2] rows left for the global insert, CTAs done
+    uint32_t* hist;           // [regions] rows per region (exact ranges)
+    uint32_t* start;          // [regions + 1] first staging row of each region (exact ranges)
+    unsigned long long* staging;  // {key, payload}, region-major
+    unsigned long long* ovf;  // [rows] {key, payload} left for the global insert
+    uint32_t* ovf_job;        // [rows] their jobs
+};
+// A table's counters (TableView::meta) and the error word, handed to the host.
+struct TableLanding {
+    uint32_t err[2];
+    unsigned long long meta[4];
 };
 // Host: group rows in ascending group order (radix sort).
 void sort_group_rows(std::vector<mgv_group_row>& v);
 inline uint32_t table_regions(const TableView& t) { return (t.nbuckets + kRegionBuckets - 1) / kRegionBuckets; }
-size_t region_scratch_bytes(uint32_t regions, uint64_t rows);
-RegionScratch carve_region_scratch(void* base, uint32_t regions, uint64_t rows);
+size_t region_zero_bytes(uint32_t regions);
+size_t region_scratch_bytes(uint32_t regions, uint64_t staged, uint64_t rows);
+RegionScratch carve_region_scratch(void* base, uint32_t regions, uint64_t staged, uint64_t rows);
+// Staging rows of each region when the ranges are fixed shares.
+uint32_t region_share(uint64_t rows, uint32_t nregions, const TableView& t, uint32_t shift);
+cudaError_t region_build_init();  // once per device: the kernels' shared memory limits
 // Items: explicit (job, rows) items, or (items == nullptr) rows [0, n) of
-// job0 cut into items of rows_per_item.  fresh: the tables hold nothing yet
-// and are not cleared beforehand; every region is written.  partitioned
-// (one job, no items): the rows arrive partitioned on the table's radix bits,
-// and are scattered by warps that sort their tiles by region.
+// job0.  exact: staging ranges from a histogram (the jobs' stage0 and cap are
+// not used).  fresh: the tables hold nothing yet and are not cleared
+// beforehand; every region is written.  land: nullable, where one table's
+// counters go afterwards.
+cudaError_t launch_build_regions(const RegionJob* d_jobs, const RegionJob& job0, uint32_t njobs,
+                                 const struct BatchItem* items, uint32_t nitems, uint64_t n, uint32_t total_regions,
+                                 uint32_t max_job_regions, const RegionScratch& sc, bool exact, bool fresh,
+                                 TableLanding* land, cudaStream_t s, Context* ctx);
 // A fresh radix-laid-out table built from a partition op's single run on its
 // radix bits (ends[p] = one past partition p's last row): per-partition
 // staging in the partition's own range, then the region build.  Only when
 // every partition slice is whole regions (region_build_partitioned_fits).
 bool region_build_partitioned_fits(const TableView& t);
 cudaError_t launch_build_regions_partitioned(const RegionJob& job, const unsigned long long* ends, uint64_t n,
-                                             const RegionScratch& sc, cudaStream_t s, Context* ctx);
-cudaError_t launch_build_regions(const RegionJob* d_jobs, const RegionJob& job0, uint32_t njobs,
-                                 const struct BatchItem* items, uint32_t nitems, uint64_t n, uint64_t rows_per_item,
-                                 uint32_t total_regions, uint32_t max_job_regions, const RegionScratch& sc,
-                                 bool fresh, bool partitioned, cudaStream_t s, Context* ctx);
+                                             const RegionScratch& sc, TableLanding* land, cudaStream_t s, Context* ctx);
+// A fresh table of at most kRegionBuckets buckets from all its rows.
+cudaError_t launch_build_small(const RegionJob& job, uint32_t n, TableLanding* land, cudaStream_t s, Context* ctx);
+cudaError_t launch_table_land(const TableView& t, TableLanding* land, cudaStream_t s, Context* ctx);
 
 struct BatchOut {  // packed result region of a query
     GroupTableView gt;

@@ -522,8 +522,10 @@ mgv_status mgv_op_create_aggregate(mgv_ctx* ctx, const mgv_aggregate_desc* d, mg
     o->agg = *d;
     mgv_status st = dev_alloc(o, (void**)&o->d_acc, 2 * sizeof(unsigned long long));
     if (st != MGV_OK) { delete o; return st; }
-    cudaError_t e = cudaMallocHost(&o->h_res, 4 * sizeof(unsigned long long));
+    cudaError_t e = cudaMallocHost(&o->h_res, 3 * sizeof(unsigned long long));
+    if (e == cudaSuccess) e = cudaHostGetDevicePointer(reinterpret_cast<void**>(&o->h_res_dev), o->h_res, 0);
     if (e != cudaSuccess) {
+        if (o->h_res) cudaFreeHost(o->h_res);
         for (void* p : o->allocs) cudaFree(p);
         delete o;
         return cuda_fail(e, "mgv_op_create_aggregate");
@@ -726,11 +728,25 @@ mgv_status mgv_op_destroy(mgv_op* o) {
     return MGV_OK;
 }
 
+// Whether an open on `s` may leave out the reset of what the last close left
+// clean: not while a graph is captured, whose replays need it every time.
+static bool skip_reset(bool clean, cudaStream_t s) {
+    if (!clean) return false;
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(s, &st) != cudaSuccess) {
+        (void)cudaGetLastError();
+        return false;
+    }
+    return st == cudaStreamCaptureStatusNone;
+}
+
 // Resets one operator's device state (at_open).
 static mgv_status op_reset(Op* o, cudaStream_t s) {
     switch (o->kind) {
         case OpKind::Aggregate:
-            MGV_CUDA_TRY(cudaMemsetAsync(o->d_acc, 0, 2 * sizeof(unsigned long long), s));
+            if (!skip_reset(o->agg_clean, s))
+                MGV_CUDA_TRY(cudaMemsetAsync(o->d_acc, 0, 2 * sizeof(unsigned long long), s));
+            o->agg_clean = true;  // until a consume or a close touches it
             o->agg_result = mgv_agg_result{0, 0};
             break;
         case OpKind::HashBuild:
@@ -754,7 +770,7 @@ static mgv_status op_reset(Op* o, cudaStream_t s) {
                 return fail(MGV_ESTATE, "hash_probe opened before its build side was closed");
             break;
         case OpKind::Groupby:
-            if (!o->gb_clean) MGV_CUDA_TRY(launch_group_reset(o->gtab, o->gb_dev_count, s, o->ctx));
+            if (!skip_reset(o->gb_clean, s)) MGV_CUDA_TRY(launch_group_reset(o->gtab, o->gb_dev_count, s, o->ctx));
             o->gb_clean = true;  // until a consume or a close touches it
             o->gb_view = nullptr;
             o->gb_n = 0;
@@ -803,16 +819,6 @@ static void hash_build_info(Op* o, const unsigned long long* m) {
 // Reads back a terminal operator's result after its stream completed.
 static mgv_status op_finish(Op* o, cudaStream_t s) {
     switch (o->kind) {
-        case OpKind::Aggregate: {
-            unsigned long long h[2];
-            MGV_CUDA_TRY(cudaMemcpyAsync(h, o->d_acc, sizeof(h), cudaMemcpyDeviceToHost, s));
-            MGV_CUDA_TRY(cudaStreamSynchronize(s));
-            o->agg_result.count = (int64_t)h[0];
-            o->agg_result.sum = (int64_t)h[1];
-            break;
-        }
-
-        case OpKind::Groupby: break;  // read back by close_groupby()
         case OpKind::Sink: {
             unsigned long long rows = 0;
             MGV_CUDA_TRY(cudaMemcpyAsync(&rows, o->sink.cursor, sizeof(rows), cudaMemcpyDeviceToHost, s));
@@ -849,14 +855,16 @@ mgv_status mgv_op_close(mgv_op* o, void* stream) {
     }
     if (!o->parent) {  // terminal: wait, check the device error word, read results
         if (o->kind == OpKind::Aggregate) {
-            // one pinned landing zone, one synchronisation
-            unsigned long long* h = o->h_res;
-            MGV_CUDA_TRY(cudaMemcpyAsync(h, o->ctx->d_err, 2 * sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
-            MGV_CUDA_TRY(cudaMemcpyAsync(h + 2, o->d_acc, 2 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, s));
+            // one kernel hands the error word and the sums to the host and leaves
+            // the sums at zero for the next open (two copies and a memset: 12 us more)
+            o->agg_clean = false;
+            MGV_CUDA_TRY(launch_agg_land(o->d_acc, o->h_res_dev, s, o->ctx));
             MGV_CUDA_TRY(cudaStreamSynchronize(s));
-            const uint32_t w[2] = {reinterpret_cast<uint32_t*>(h)[0], reinterpret_cast<uint32_t*>(h)[1]};
-            o->agg_result.count = (int64_t)h[2];
-            o->agg_result.sum = (int64_t)h[3];
+            o->agg_clean = true;
+            const unsigned long long* h = o->h_res;
+            const uint32_t w[2] = {(uint32_t)h[0], (uint32_t)(h[0] >> 32)};
+            o->agg_result.count = (int64_t)h[1];
+            o->agg_result.sum = (int64_t)h[2];
             return report_device_error(o->ctx, w, s);
         }
         if (o->kind == OpKind::Groupby) return close_groupby(o, s);
@@ -1103,6 +1111,7 @@ static mgv_status consume_cols(Op* head, const int32_t* const* cols, uint32_t nc
             const int32_t ca = term->agg.sum_col_a, cb = term->agg.sum_col_b;
             if (!ref_ok(ca) || !ref_ok(cb)) return fail(MGV_EINVAL, "aggregate column not in input");
             if (n == 0) return MGV_OK;
+            term->agg_clean = false;
             // select -> aggregate: the masked fold, unless the context asks
             // for the warp-ballot compaction of the chain kernel
             if (!probe && !(sel && ctx->tuning.select_compact)) {

@@ -146,6 +146,20 @@ cudaError_t launch_select_agg(const int32_t* filt, int32_t bound, bool has_sel, 
     }
 }
 
+__global__ void k_agg_land(unsigned long long* acc, unsigned long long* land, const uint32_t* err) {
+    if (threadIdx.x != 0) return;
+    land[0] = (unsigned long long)err[1] << 32 | err[0];
+    land[1] = acc[0];
+    land[2] = acc[1];
+    acc[0] = acc[1] = 0;
+}
+
+cudaError_t launch_agg_land(unsigned long long* acc, unsigned long long* land, cudaStream_t s, Context* ctx) {
+    k_agg_land<<<1, 32, 0, s>>>(acc, land, ctx->d_err);
+    ctx->launches++;
+    return cudaGetLastError();
+}
+
 // ---------------------------------------------------------------------------
 // hash build  (hashjoin_builder::consume_warp, src/operators/hashjoin.cu:40-60)
 //

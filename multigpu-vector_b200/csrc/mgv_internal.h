@@ -139,6 +139,8 @@ struct Op {
     mgv_aggregate_desc agg{};
     unsigned long long* d_acc = nullptr;    // [count, sum]
     unsigned long long* h_res = nullptr;    // pinned: the error word and the results read back at close
+    unsigned long long* h_res_dev = nullptr;  // the same as the device addresses it (aggregate)
+    bool agg_clean = false;                 // d_acc is zero on the device (a close leaves it so)
     mgv_agg_result agg_result{};
     // hash build
     mgv_hash_build_desc hb{};
@@ -218,6 +220,8 @@ cudaError_t launch_fill_u64(unsigned long long* p, uint64_t n, unsigned long lon
 cudaError_t launch_select_agg(const int32_t* filt, int32_t bound, bool has_sel, const int32_t* a,
                               const int32_t* b, uint64_t n, unsigned long long* acc, cudaStream_t s,
                               Context* ctx);
+// {error word, count, sum} to the host (pinned, mapped), and the sums back to zero.
+cudaError_t launch_agg_land(unsigned long long* acc, unsigned long long* land, cudaStream_t s, Context* ctx);
 cudaError_t launch_build(const int32_t* keys, const int32_t* pays, const int32_t* filt,
                          int32_t bound, bool has_sel, uint64_t n, const TableView& t,
                          cudaStream_t s, Context* ctx);

@@ -40,6 +40,29 @@ constexpr uint32_t kWaitTries = 1u << 24;
 template <int R>
 constexpr int queue_len() { return 32 * (R + 1) <= 160 ? 256 : 512; }
 
+// The tiles of a probe: `tiles` of them from row `head` on, where the keys are
+// 16-byte aligned, as the bulk copies need it.  The payloads there start
+// `skew` rows past such a boundary; a stage then takes the 16 bytes around both
+// ends of its tile, which lie inside the column: `head` and `tiles` see to it.
+// An aligned pair of columns has head 0 and skew 0.
+struct TileCut {
+    uint64_t tiles;
+    uint32_t head;
+    uint32_t skew;
+};
+
+TileCut cut_tiles(const int32_t* keys, const int32_t* pays, uint64_t n, uint64_t tile) {
+    const uint32_t k = ((uintptr_t)keys & 15u) / 4, p = ((uintptr_t)pays & 15u) / 4;
+    TileCut c;
+    c.head = (4 - k) & 3u;
+    c.skew = pays ? (p + c.head) & 3u : 0;
+    if (c.skew > c.head) c.head += 4;
+    const uint64_t outside = c.head + (c.skew ? 4 - c.skew : 0);
+    c.tiles = n > outside ? (n - outside) / tile : 0;
+    if (c.tiles == 0) c.head = c.skew = 0;  // every row from global memory
+    return c;
+}
+
 struct Acc {
     uint32_t cnt;            // matches of this thread (fits: rows per thread < 2^32)
     unsigned long long sum;  // two's-complement int64
@@ -295,22 +318,28 @@ __global__ void __launch_bounds__(kThreads, MB)
 // stage is released once its folds are done.  Continuations are served by
 // continuation-only rounds (one load per lane) whenever the queue holds a
 // batch, which also keeps room for a tile's appends.
-template <int R, int S, int MB, bool UNIQUE, bool ADD_BP, bool ADD_PP, bool RADIX, bool KO = false>
+// SKEW: the columns are slices that do not start on 16-byte boundaries
+// (TileCut); apart from the aligned form, which 40 us of a 335 us probe of 2^26
+// rows depend on (its stages on 128-byte boundaries, its one ragged round).
+template <int R, int S, int MB, bool UNIQUE, bool ADD_BP, bool ADD_PP, bool RADIX, bool KO = false, bool SKEW = false>
 __global__ void __launch_bounds__(kThreads, MB)
     k_probe_agg_pipe(const int32_t* __restrict__ keys, const int32_t* __restrict__ pays, uint64_t n, TableView t,
-                     unsigned long long* acc, uint32_t* err) {
+                     unsigned long long* acc, uint32_t* err, TileCut cut) {
     constexpr int T = kConsumerWarps * 32 * R;  // rows per tile
     constexpr int Q = queue_len<R>();
     constexpr uint32_t kRoomLimit = (uint32_t)(Q - 32 * (R + 1));
     extern __shared__ __align__(128) unsigned char smem_raw[];
     int32_t* sk = reinterpret_cast<int32_t*>(smem_raw);
     int32_t* sp = sk + S * T;
-    int32_t* qbase = sp + (ADD_PP ? S * T : 0);
+    constexpr int PT = SKEW ? T + 32 : T;  // rows of payload space in a stage
+    int32_t* qbase = sp + (ADD_PP ? S * PT : 0);
     uint32_t* tails = reinterpret_cast<uint32_t*>(qbase + 3 * kConsumerWarps * Q);
     uint64_t* full = reinterpret_cast<uint64_t*>(tails + kConsumerWarps);
     uint64_t* empty = full + S;
 
-    const uint64_t nfull = n / T;
+    const uint64_t nfull = SKEW ? cut.tiles : n / T;
+    const uint32_t head = SKEW ? cut.head : 0u, skew = SKEW ? cut.skew : 0u;
+    const uint32_t pay_bytes = (uint32_t)T * sizeof(int32_t) + (skew ? 16u : 0u);
     const uint64_t my_tiles = nfull > blockIdx.x ? (nfull - blockIdx.x + gridDim.x - 1) / gridDim.x : 0;
     const uint32_t tile_bytes = (uint32_t)T * sizeof(int32_t);
     const int warp = threadIdx.x / 32;
@@ -342,9 +371,10 @@ __global__ void __launch_bounds__(kThreads, MB)
                     break;
                 }
                 const uint64_t tile = blockIdx.x + i * gridDim.x;
-                mbar_expect_tx(&full[s], ADD_PP ? 2 * tile_bytes : tile_bytes);
-                bulk_g2s_hint(sk + s * T, keys + tile * T, tile_bytes, &full[s], stream_policy);
-                if (ADD_PP) bulk_g2s_hint(sp + s * T, pays + tile * T, tile_bytes, &full[s], stream_policy);
+                mbar_expect_tx(&full[s], ADD_PP ? tile_bytes + pay_bytes : tile_bytes);
+                bulk_g2s_hint(sk + s * T, keys + head + tile * T, tile_bytes, &full[s], stream_policy);
+                if (ADD_PP)
+                    bulk_g2s_hint(sp + s * PT, pays + head + tile * T - skew, pay_bytes, &full[s], stream_policy);
             }
             const uint64_t lo = i > (uint64_t)S ? i - S : 0;
             for (uint64_t j = lo; j < i; ++j) mbar_wait_bounded(&full[j % S], (uint32_t)((j / S) & 1), kWaitTries);
@@ -382,7 +412,7 @@ __global__ void __launch_bounds__(kThreads, MB)
             // room for this tile's appends; the rounds use their own registers
             make_room<R, Q, UNIQUE, ADD_BP, ADD_PP, RADIX, KO>(q, t, a, kRoomLimit);
             const int32_t* rk = sk + s * T + row0;
-            const int32_t* rp = sp + s * T + row0;
+            const int32_t* rp = sp + s * PT + skew + row0;
             const int32_t* nk = sk + s1 * T + row0;
             uint32_t dep = 0;
 #pragma unroll
@@ -406,14 +436,24 @@ __global__ void __launch_bounds__(kThreads, MB)
             }
         }
         if (ok && blockIdx.x == gridDim.x - 1) {
-            // rows of the last partial tile, straight from global memory
-            const uint64_t base = nfull * T + (uint64_t)row0;
-            uint32_t valid = 0;
+            // rows outside the tiles, straight from global memory: after the last
+            // tile and, of a slice, up to 7 before the first (and then up to 3 more
+            // than a tile after it)
+            uint64_t lo = SKEW && head ? 0 : head + nfull * T, hi = SKEW && head ? head : n;
+            do {
+                const uint64_t base = lo + (uint64_t)row0;
+                uint32_t valid = 0;
 #pragma unroll
-            for (int r = 0; r < R; ++r) valid |= (uint32_t)(base + 32 * r < n) << r;
-            make_room<R, Q, UNIQUE, ADD_BP, ADD_PP, RADIX, KO>(q, t, a, kRoomLimit);
-            round<R, Q, UNIQUE, ADD_BP, ADD_PP, RADIX, KO>(keys + base, ADD_PP ? pays + base : nullptr, valid, q, false,
-                                                           t, a);
+                for (int r = 0; r < R; ++r) valid |= (uint32_t)(base + 32 * r < hi) << r;
+                make_room<R, Q, UNIQUE, ADD_BP, ADD_PP, RADIX, KO>(q, t, a, kRoomLimit);
+                round<R, Q, UNIQUE, ADD_BP, ADD_PP, RADIX, KO>(keys + base, ADD_PP ? pays + base : nullptr, valid, q,
+                                                               false, t, a);
+                lo += T;
+                if (SKEW && head && hi == head) {
+                    lo = head + nfull * T;
+                    hi = n;
+                }
+            } while (SKEW && lo < hi);
         }
         // drain the continuation queue
         make_room<R, Q, UNIQUE, ADD_BP, ADD_PP, RADIX, KO>(q, t, a, 0u);
@@ -421,63 +461,71 @@ __global__ void __launch_bounds__(kThreads, MB)
     block_accumulate2<kThreads>((unsigned long long)a.cnt, a.sum, acc);
 }
 
-template <int R, int S, int MB, bool UNIQUE, bool ADD_BP, bool ADD_PP, bool RADIX, bool KO = false>
+template <int R, int S, int MB, bool UNIQUE, bool ADD_BP, bool ADD_PP, bool RADIX, bool KO = false, bool SKEW = false>
 cudaError_t launch_v(const int32_t* keys, const int32_t* pays, uint64_t n, const TableView& t,
                      unsigned long long* acc, int ctas_per_sm, cudaStream_t s, Context* ctx) {
-    // probe_kernel 0 (auto) and 3: the software-pipelined consumer rounds
-    // (measured faster); 2: the plain rounds
-    auto k = ctx->tuning.probe_kernel == 2 ? k_probe_agg_ws<R, S, MB, UNIQUE, ADD_BP, ADD_PP, RADIX, KO>
-                                           : k_probe_agg_pipe<R, S, MB, UNIQUE, ADD_BP, ADD_PP, RADIX, KO>;
     constexpr int T = kConsumerWarps * 32 * R;
-    const size_t smem = (size_t)(ADD_PP ? 2 : 1) * S * T * sizeof(int32_t) +
+    const TileCut cut = SKEW ? cut_tiles(keys, ADD_PP ? pays : nullptr, n, T) : TileCut{n / T, 0, 0};
+    const size_t smem = (size_t)S * ((ADD_PP ? 2 * T : T) + (SKEW ? 32 : 0)) * sizeof(int32_t) +
                         (size_t)3 * kConsumerWarps * queue_len<R>() * sizeof(int32_t) +
                         kConsumerWarps * sizeof(uint32_t) + 2 * S * sizeof(uint64_t);
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-    int per_sm = 0;
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, kThreads, smem);
-    if (e != cudaSuccess) return e;
-    if (per_sm < 1) per_sm = 1;
-    if (ctas_per_sm > 0 && ctas_per_sm < per_sm) per_sm = ctas_per_sm;
-    uint64_t grid = (uint64_t)per_sm * ctx->prop.multiProcessorCount;
-    const uint64_t nfull = n / T;
-    if (grid > nfull) grid = nfull ? nfull : 1;
-    k<<<(int)grid, kThreads, smem, s>>>(keys, pays, n, t, acc, ctx->d_err);
-    ctx->launches++;
-    return cudaGetLastError();
+    auto launch = [&](auto k, auto... extra) -> cudaError_t {
+        cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e != cudaSuccess) return e;
+        int per_sm = 0;
+        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, kThreads, smem);
+        if (e != cudaSuccess) return e;
+        if (per_sm < 1) per_sm = 1;
+        if (ctas_per_sm > 0 && ctas_per_sm < per_sm) per_sm = ctas_per_sm;
+        uint64_t grid = (uint64_t)per_sm * ctx->prop.multiProcessorCount;
+        if (grid > cut.tiles) grid = cut.tiles ? cut.tiles : 1;
+        k<<<(int)grid, kThreads, smem, s>>>(keys, pays, n, t, acc, ctx->d_err, extra...);
+        ctx->launches++;
+        return cudaGetLastError();
+    };
+    // probe_kernel 0 (auto) and 3: the software-pipelined consumer rounds
+    // (measured faster); 2: the plain rounds
+    if constexpr (!SKEW)
+        if (ctx->tuning.probe_kernel == 2) return launch(k_probe_agg_ws<R, S, MB, UNIQUE, ADD_BP, ADD_PP, RADIX, KO>);
+    return launch(k_probe_agg_pipe<R, S, MB, UNIQUE, ADD_BP, ADD_PP, RADIX, KO, SKEW>, cut);
 }
 
-template <int R, int S, int MB, bool UNIQUE, bool RADIX>
+template <int R, int S, int MB, bool UNIQUE, bool RADIX, bool SKEW>
 cudaError_t launch_mode_r(const int32_t* keys, const int32_t* pays, uint64_t n, const TableView& t, uint32_t mode,
                           unsigned long long* acc, int ctas, cudaStream_t s, Context* ctx) {
     switch (mode) {
-        case 0: return launch_v<R, S, MB, UNIQUE, false, false, RADIX>(keys, pays, n, t, acc, ctas, s, ctx);
-        case 1: return launch_v<R, S, MB, UNIQUE, true, false, RADIX>(keys, pays, n, t, acc, ctas, s, ctx);
-        case 2: return launch_v<R, S, MB, UNIQUE, false, true, RADIX>(keys, pays, n, t, acc, ctas, s, ctx);
-        default: return launch_v<R, S, MB, UNIQUE, true, true, RADIX>(keys, pays, n, t, acc, ctas, s, ctx);
+        case 0: return launch_v<R, S, MB, UNIQUE, false, false, RADIX, false, SKEW>(keys, pays, n, t, acc, ctas, s, ctx);
+        case 1: return launch_v<R, S, MB, UNIQUE, true, false, RADIX, false, SKEW>(keys, pays, n, t, acc, ctas, s, ctx);
+        case 2: return launch_v<R, S, MB, UNIQUE, false, true, RADIX, false, SKEW>(keys, pays, n, t, acc, ctas, s, ctx);
+        default: return launch_v<R, S, MB, UNIQUE, true, true, RADIX, false, SKEW>(keys, pays, n, t, acc, ctas, s, ctx);
     }
 }
 
-template <int R, int S, int MB, bool UNIQUE>
+template <int R, int S, int MB, bool UNIQUE, bool SKEW = false>
 cudaError_t launch_mode(const int32_t* keys, const int32_t* pays, uint64_t n, const TableView& t, uint32_t mode,
                         unsigned long long* acc, int ctas, cudaStream_t s, Context* ctx) {
-    if (t.radix_mask != 0) return launch_mode_r<R, S, MB, UNIQUE, true>(keys, pays, n, t, mode, acc, ctas, s, ctx);
-    return launch_mode_r<R, S, MB, UNIQUE, false>(keys, pays, n, t, mode, acc, ctas, s, ctx);
+    if (t.radix_mask != 0) return launch_mode_r<R, S, MB, UNIQUE, true, SKEW>(keys, pays, n, t, mode, acc, ctas, s, ctx);
+    return launch_mode_r<R, S, MB, UNIQUE, false, SKEW>(keys, pays, n, t, mode, acc, ctas, s, ctx);
 }
 
 }  // namespace
 
-// Returns cudaErrorNotSupported when this kernel does not apply (columns
-// not 16-byte aligned); the caller then uses the register-prefetch kernel.
+// Returns cudaErrorNotSupported when this kernel does not apply (columns not
+// aligned to their rows); the caller then uses the register-prefetch kernel.
+// Column slices that start at any row take this one: 2 M rows of such a slice
+// against a table with repeated keys, 86 us through the register prefetch.
 cudaError_t launch_probe_agg_staged(const int32_t* keys, const int32_t* pays, uint64_t n, const TableView& t,
                                     bool unique, uint32_t sum_mode, unsigned long long* acc, cudaStream_t s,
                                     Context* ctx) {
-    if (((uintptr_t)keys & 15u) || ((uintptr_t)pays & 15u)) return cudaErrorNotSupported;
+    if (((uintptr_t)keys & 3u) || ((uintptr_t)pays & 3u)) return cudaErrorNotSupported;
     const uint32_t mode = (sum_mode & 1u) | ((sum_mode & 2u) && pays ? 2u : 0u);
+    const bool skew = ((uintptr_t)keys & 15u) || ((mode & 2u) && ((uintptr_t)pays & 15u));
     if (t.key_only) {  // eight keys per bucket, payloads 0: the default shape only
         const bool radix = t.radix_mask != 0, pp = (mode & 2u) != 0;
         const int ctas = (int)ctx->tuning.probe_ctas_per_sm;
-#define MGV_KO(U, P, X) return launch_v<4, 4, 3, U, false, P, X, true>(keys, pays, n, t, acc, ctas, s, ctx)
+#define MGV_KO(U, P, X)                                                                                     \
+    return skew ? launch_v<4, 4, 3, U, false, P, X, true, true>(keys, pays, n, t, acc, ctas, s, ctx)       \
+                : launch_v<4, 4, 3, U, false, P, X, true>(keys, pays, n, t, acc, ctas, s, ctx)
         if (unique) {
             if (pp) { if (radix) MGV_KO(true, true, true); MGV_KO(true, true, false); }
             if (radix) MGV_KO(true, false, true);
@@ -490,6 +538,9 @@ cudaError_t launch_probe_agg_staged(const int32_t* keys, const int32_t* pays, ui
     }
     const mgv_tuning& tu = ctx->tuning;
     const int ctas = (int)tu.probe_ctas_per_sm;
+    if (skew)  // slices: the default shape only
+        return unique ? launch_mode<4, 4, 3, true, true>(keys, pays, n, t, mode, acc, ctas, s, ctx)
+                      : launch_mode<4, 4, 3, false, true>(keys, pays, n, t, mode, acc, ctas, s, ctx);
     const int st = tu.probe_stages <= 2 ? 2 : tu.probe_stages <= 4 ? 4 : 6;
     // Register budgets: R = 4 at 2, 3 or 4 CTAs per SM (3 and 4 when
     // probe_ctas_per_sm asks for them), R = 8 at 1 (at 2 it spills).

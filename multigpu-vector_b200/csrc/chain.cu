@@ -4,10 +4,10 @@
 //
 // one kernel per consume call.  Warp-ballot select as in
 // unstable_select::consume_warp (src/operators/select3.cu:19-85): each warp
-// takes 512-row windows (16 filter loads per lane in flight), evaluates the
+// takes 256-row windows (8 filter loads per lane in flight), evaluates the
 // predicate and compacts the offsets of the qualifying rows with
-// __ballot_sync / __popc into a per-warp shared-memory ring of 1024 entries.
-// Every 128 offsets form a vector whose carried columns -- only those the
+// __ballot_sync / __popc into a per-warp shared-memory ring of 512 entries.
+// Every 64 offsets form a vector whose carried columns -- only those the
 // rest of the chain reads -- are gathered and handed to the probe and the
 // terminal (the reference's parent->consume_warp(x, 128)).
 //
@@ -36,10 +36,17 @@
 
 namespace mgv {
 
-constexpr int kChainBlock = 512;  // 16 warps: one CTA per SM with the largest group table
+// 32 warps, one CTA per SM with the largest group table, and two rows per lane
+// in a vector.  A vector is a string of dependent latencies (column gathers,
+// buckets, group lookup, shared atomics), so warps count more than rows per
+// warp: 64-query batch 1492 us with 16 warps and four rows per lane, 1165 us
+// here, 1343 us with 32 warps and one row; shared scan 245 / 176 / 150 us.
+constexpr int kChainBlock = 1024;
 constexpr int kChainWarps = kChainBlock / 32;
-constexpr int kWinRows = 512;  // rows per warp per select window: 16 loads per lane in flight
-constexpr int kIdRing = 1024;  // per-warp ring of qualifying row offsets (>= kWinRows + 127)
+constexpr int kVecRows = 2;            // rows per lane of a vector
+constexpr uint32_t kVec = 32 * kVecRows;
+constexpr int kWinRows = 256;  // rows per warp per select window: 8 loads per lane in flight
+constexpr int kIdRing = 512;   // per-warp ring of qualifying row offsets (>= kWinRows + kVec - 1)
 constexpr int kMaxTermSlots = 3;  // carried columns of an aggregate / group-by chain: key + 2 references
 constexpr size_t kRingBytes = (size_t)kChainWarps * kIdRing * sizeof(uint32_t);
 
@@ -101,8 +108,9 @@ struct SinkStage {
 
 // Writes the `n` staged rows of a warp (n <= kSinkStage) to the sink: output
 // column c is input column a.ref[c] of the staged row, or its build payload.
-// Consecutive lanes write consecutive rows, one column after another.
-__device__ __noinline__ void sink_flush(const ChainDev& a, const SinkStage& st, uint32_t n, uint32_t* err) {
+// Consecutive lanes write consecutive rows, one column after another.  Inlined:
+// as a call it costs the probe's registers (8 M rows 167 us against 137 us).
+__device__ __forceinline__ void sink_flush(const ChainDev& a, const SinkStage& st, uint32_t n, uint32_t* err) {
     const SinkView& s = a.sink;
     const uint32_t lane = lane_id();
     __syncwarp();
@@ -429,7 +437,7 @@ __device__ __forceinline__ uint32_t cell_range_of(const CellCtx& cc, uint32_t m,
 // Value of carried slot `slot` (a run-time index) from the registers of a
 // vector; j is a compile-time row position after unrolling.
 template <int NS>
-__device__ __forceinline__ int32_t pick_slot(const int32_t (&v)[NS][4], int32_t slot, int j) {
+__device__ __forceinline__ int32_t pick_slot(const int32_t (&v)[NS][kVecRows], int32_t slot, int j) {
     int32_t r = 0;
 #pragma unroll
     for (int c = 0; c < NS; ++c)
@@ -440,11 +448,11 @@ __device__ __forceinline__ int32_t pick_slot(const int32_t (&v)[NS][4], int32_t 
 // Windows of kWinRows rows of [row_lo, row_hi) (fewer than 2^32 rows), this
 // warp taking windows win_first, win_first + win_stride, ...
 //
-// A window is filtered with 16 independent coalesced loads per lane (one
+// A window is filtered with 8 independent coalesced loads per lane (one
 // 128-byte warp load each, all in flight together), and the offsets of its
 // qualifying rows are compacted with __ballot_sync / __popc into the warp's
-// shared ring, in row order.  Every 128 offsets form a vector: its carried
-// columns are gathered into registers (4 rows per lane, all loads
+// shared ring, in row order.  Every 64 offsets form a vector: its carried
+// columns are gathered into registers (2 rows per lane, all loads
 // independent), its keys probed, and its rows handed to the terminal.  Only
 // qualifying rows' columns are ever loaded.
 template <bool SEL, bool PROBE, int TERM, bool FIXED = false>
@@ -470,22 +478,22 @@ __device__ __forceinline__ void chain_windows(const ChainDev& a, bool unique, ui
 
     // sink: room in the staging for one match per row of a vector
     auto make_room = [&]() {
-        if (staged > kSinkStage - 128) {
+        if (staged > kSinkStage - kVec) {
             sink_flush(a, *stage, staged, err);
             staged = 0;
         }
     };
 
-    // push `cnt` (<= 128) rows: the ring's offsets from `start` on, or without
+    // push `cnt` (<= kVec) rows: the ring's offsets from `start` on, or without
     // a select the rows from `start` on themselves
     auto push_vector = [&](uint32_t start, uint32_t cnt) {
         __syncwarp();
         if (TERM == kTermSink) make_room();
-        uint32_t rid[4];
-        uint32_t rng[4];  // shared scan: each row's filter range
-        bool in[4];
+        uint32_t rid[kVecRows];
+        uint32_t rng[kVecRows];  // shared scan: each row's filter range
+        bool in[kVecRows];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
+        for (int j = 0; j < kVecRows; ++j) {
             const uint32_t idx = j * 32 + lane;
             in[j] = idx < cnt;
             rid[j] = SEL ? ids[(start + idx) & (kIdRing - 1)] : start + idx;
@@ -495,13 +503,13 @@ __device__ __forceinline__ void chain_windows(const ChainDev& a, bool unique, ui
                 rid[j] &= (1u << kCellRowBits) - 1u;
             }
         }
-        int32_t v[NS][4];
+        int32_t v[NS][kVecRows];
 #pragma unroll
         for (int c = 0; c < NS; ++c) {
             const bool carried = (uint32_t)c < nslots;
             const int32_t* col = carried ? slot_col(c) + row_lo : nullptr;
 #pragma unroll
-            for (int j = 0; j < 4; ++j)  // a sink's flush reads the key again: no evict-first for it
+            for (int j = 0; j < kVecRows; ++j)  // a sink's flush reads the key again: no evict-first for it
                 v[c][j] = !(carried && in[j])  ? 0
                           : TERM == kTermSink ? __ldg(col + rid[j])
                                               : ld_stream1(col + rid[j], stream_policy);
@@ -544,21 +552,21 @@ __device__ __forceinline__ void chain_windows(const ChainDev& a, bool unique, ui
         };
         if (!PROBE) {
 #pragma unroll
-            for (int j = 0; j < 4; ++j) emit(in[j], j, 0);
+            for (int j = 0; j < kVecRows; ++j) emit(in[j], j, 0);
         } else {
-            // Rounds over the four rows' runs: every round examines one bucket
+            // Rounds over the rows' runs: every round examines one bucket
             // per row still walking and emits its matches; the rows whose run
             // continues past a full bucket then load their next buckets
             // together, so a round costs one memory latency for all of them.
             const unsigned long long* __restrict__ slots = a.table.slots;
             const uint32_t nbuckets = a.table.nbuckets;
-            uint32_t w[4][8];
-            uint32_t b[4];
-            int32_t key[4];
-            bool live[4];
+            uint32_t w[kVecRows][8];
+            uint32_t b[kVecRows];
+            int32_t key[kVecRows];
+            bool live[kVecRows];
             bool reserved_any = false;
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
+            for (int j = 0; j < kVecRows; ++j) {
                 key[j] = pick_slot<NS>(v, probe_slot, j);
                 live[j] = in[j] && key[j] != kEmptyKey;
                 reserved_any |= in[j] && key[j] == kEmptyKey;
@@ -567,7 +575,7 @@ __device__ __forceinline__ void chain_windows(const ChainDev& a, bool unique, ui
                 const uint32_t side_n =
                     (uint32_t)min((unsigned long long)a.table.meta[0], (unsigned long long)a.table.side_cap);
 #pragma unroll
-                for (int j = 0; j < 4; ++j) {
+                for (int j = 0; j < kVecRows; ++j) {
                     const bool r = in[j] && key[j] == kEmptyKey;
                     if (__any_sync(0xffffffffu, r))
                         for (uint32_t i = 0; i < side_n; ++i) {
@@ -577,14 +585,14 @@ __device__ __forceinline__ void chain_windows(const ChainDev& a, bool unique, ui
                 }
             }
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
+            for (int j = 0; j < kVecRows; ++j) {
                 b[j] = home_bucket(key[j], a.table);
                 if (live[j]) ld_bucket(slots + 4ull * b[j], w[j]);
             }
             const bool ko = a.table.key_only != 0;  // eight keys per bucket, payloads 0
             for (uint32_t round = 0; round <= nbuckets; ++round) {
 #pragma unroll
-                for (int j = 0; j < 4; ++j) {
+                for (int j = 0; j < kVecRows; ++j) {
                     const uint32_t k = (uint32_t)key[j];
                     if (TERM == kTermSink) {
                         // the bucket's matching slots as bits, emitted one per lane and
@@ -643,9 +651,12 @@ __device__ __forceinline__ void chain_windows(const ChainDev& a, bool unique, ui
                         live[j] = live[j] && w[j][6] != (uint32_t)kEmptyKey;
                     }
                 }
-                if (!__any_sync(0xffffffffu, live[0] || live[1] || live[2] || live[3])) break;
+                bool any = false;
 #pragma unroll
-                for (int j = 0; j < 4; ++j)
+                for (int j = 0; j < kVecRows; ++j) any |= live[j];
+                if (!__any_sync(0xffffffffu, any)) break;
+#pragma unroll
+                for (int j = 0; j < kVecRows; ++j)
                     if (live[j]) {
                         b[j] = (b[j] + 1 == nbuckets) ? 0u : b[j] + 1;
                         ld_bucket(slots + 4ull * b[j], w[j]);
@@ -657,13 +668,13 @@ __device__ __forceinline__ void chain_windows(const ChainDev& a, bool unique, ui
 
     const int32_t* __restrict__ fcol = SEL ? a.cols[a.sel_col] + row_lo : nullptr;
     const uint64_t nwin = (len + kWinRows - 1) / kWinRows;
-    uint32_t head = 0, fill = 0;  // fill < 128 between windows
+    uint32_t head = 0, fill = 0;  // fill < kVec between windows
     for (uint64_t win = win_first; win < nwin; win += win_stride) {
         const uint32_t r0 = (uint32_t)win * kWinRows;
         if (!SEL) {  // every row qualifies: no ring
             const uint32_t r1 = min(len - r0, (uint32_t)kWinRows) + r0;
 #pragma unroll 1
-            for (uint32_t r = r0; r < r1; r += 128) push_vector(r, min(r1 - r, 128u));
+            for (uint32_t r = r0; r < r1; r += kVec) push_vector(r, min(r1 - r, kVec));
         }
         if (SEL) {
             int32_t f[kWinRows / 32];
@@ -684,10 +695,10 @@ __device__ __forceinline__ void chain_windows(const ChainDev& a, bool unique, ui
                 }
                 fill += __popc(m);
             }
-            while (fill >= 128) {
-                push_vector(head, 128);
-                head = (head + 128) & (kIdRing - 1);
-                fill -= 128;
+            while (fill >= kVec) {
+                push_vector(head, kVec);
+                head = (head + kVec) & (kIdRing - 1);
+                fill -= kVec;
             }
         }
     }
@@ -698,7 +709,8 @@ __device__ __forceinline__ void chain_windows(const ChainDev& a, bool unique, ui
 // Shared layout of k_chain: [id rings (a select's) | group table or sink staging].
 // A sink chain keeps no group table and reads its output columns in the
 // flush, so its warps need fewer registers: two CTAs of 12 warps per SM hide
-// more of the bucket reads' latency than one of 16.
+// more of the bucket reads' latency than one of 16 (of 8 and 16 warps: 215 and
+// 185 us against 167 us).
 constexpr int kSinkBlock = 384;
 template <int TERM>
 constexpr int chain_block() { return TERM == kTermSink ? kSinkBlock : kChainBlock; }

@@ -256,10 +256,9 @@ __global__ void __launch_bounds__(kRBlock) k_region_scatter(const RegionJob* __r
 // ---- sorted tiles -------------------------------------------------------------
 
 constexpr int kTileBlock = 512;
-// Rows per thread, held in registers from load to placement ({key, payload}
-// rows: 16 spill 170 bytes at 64 registers).
+// Rows per thread, held in registers from load to placement.
 template <bool KO>
-constexpr int tile_rows() { return KO ? 16 : 12; }
+constexpr int tile_rows() { return 16; }
 template <bool KO>
 constexpr uint32_t tile_size() { return kTileBlock * tile_rows<KO>(); }
 constexpr uint32_t kTileRegions = 4096;   // most regions a tile sorts: runs of two rows on average
@@ -295,18 +294,13 @@ __device__ __forceinline__ TileSpace<KO> tile_space(unsigned char* base, uint32_
     return s;
 }
 
-// The rows of a tile with the reserved key, to the side list (rare: the rows
-// are read again here, so that the tile's own code keeps no insert).  Returns
-// how many were this thread's.
-__device__ __noinline__ uint32_t side_list_rows(const RegionJob& job, uint64_t lo, uint64_t hi, uint32_t* err) {
-    uint32_t rows = 0;
-    for (uint64_t i = lo + threadIdx.x; i < hi; i += kTileBlock) {
-        if (__ldg(job.keys + i) != kEmptyKey || (job.filt && __ldg(job.filt + i) > job.bound)) continue;
-        bool dup, ok;
-        table_insert(job.t, kEmptyKey, job.pays ? __ldg(job.pays + i) : 0, err, dup, ok);
-        ++rows;
-    }
-    return rows;
+// One build row with the reserved key: the side list (its duplicates are seen
+// from its count), as table_insert does it, without the rest of the insert.
+__device__ __forceinline__ void side_list_row(const TableView& t, int32_t pay, uint32_t* err) {
+    const unsigned long long i = atomicAdd(t.meta + 0, 1ull);
+    atomicAdd(t.meta + 1, (unsigned long long)(long long)pay);
+    if (i < t.side_cap) t.side_pay[i] = pay;
+    else set_error(err, kDevTableFull, 1);
 }
 
 // Rows [lo, hi) (at most tile_size) of a job to their regions: ranks by shared
@@ -344,9 +338,13 @@ __device__ __forceinline__ void sort_tile(const RegionJob& job, const TileSpace<
 #pragma unroll
     for (int u = 0; u < tile_rows<KO>(); ++u)
         if (at[u] != ~0u) at[u] |= atomicAdd(ts.off + (at[u] >> 16) * ts.copies + copy, 1u);
-    if (reserved) {
-        const uint32_t rows = side_list_rows(job, lo, hi, err);
-        if (side_rows && rows) atomicAdd(side_rows, rows);
+    if (reserved) {  // rare: the rows are read again, so that the common path holds nothing for them
+#pragma unroll 1
+        for (uint32_t i = threadIdx.x; i < n; i += kTileBlock) {
+            if (__ldg(keys + i) != kEmptyKey || (filt && __ldg(filt + i) > bound)) continue;
+            side_list_row(job.t, job.pays ? __ldg(job.pays + lo + i) : 0, err);
+            if (side_rows) atomicAdd(side_rows, 1u);
+        }
     }
     __syncthreads();
     const uint32_t total = block_exclusive_scan<kTileBlock>(ts.off, regions * ts.copies);

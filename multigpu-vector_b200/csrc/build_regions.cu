@@ -46,7 +46,7 @@ namespace mgv {
 namespace {
 
 constexpr int kRBlock = 512;       // histogram / scatter CTA
-constexpr int kRBuildBlock = 512;  // largest region build CTA: a thread per 4 buckets
+constexpr int kRBuildBlock = 512;  // region build CTA: a thread per 2 to 4 buckets
 constexpr int kScanBlock = 1024;
 
 // The job of item / region lookups, cached in shared memory by the caller.
@@ -537,9 +537,12 @@ __device__ __forceinline__ void clear_table(unsigned long long* tab, uint32_t nb
     for (uint32_t w = threadIdx.x; w < 2 * nb; w += blockDim.x) reinterpret_cast<uint4*>(tab)[w] = empty;
 }
 
-// Staging rows per thread in one load batch: at load factor 0.5 all of a region's.
+// Staging rows per thread in one load batch.  Few: at 40 registers (three CTAs)
+// the whole region's rows, 16 keys or 8 {key, payload}, spilled, and with the
+// tables in shared memory there is hardly an L1 for spills (2^22 {key, payload}
+// rows 51 -> 41 us, 2^24 keys 107 -> 92 us).
 template <bool KO>
-constexpr int region_batch() { return KO ? 16 : 8; }
+constexpr int region_batch() { return KO ? 4 : 2; }
 
 // A region's staging rows.
 struct RegionRows {
@@ -872,7 +875,7 @@ static cudaError_t build_staged(const RegionJob* d_jobs, const RegionJob& job0, 
     const bool ko = job0.t.key_only != 0;
     const void* kb = ko ? (const void*)k_region_build<true> : (const void*)k_region_build<false>;
     const size_t smem = region_smem(shift);
-    const int block = (int)std::min((uint32_t)kRBuildBlock, (1u << shift) / 4);
+    const int block = (int)std::min((uint32_t)kRBuildBlock, (1u << shift) / 2);
     const int grid = (int)std::min<uint64_t>(regions, (uint64_t)occupancy_grid(kb, block, smem, ctx));
     if (ko) k_region_build<true><<<grid, block, smem, s>>>(d_jobs, job0, njobs, regions, out, fresh ? 1u : 0u, ctx->d_err);
     else k_region_build<false><<<grid, block, smem, s>>>(d_jobs, job0, njobs, regions, out, fresh ? 1u : 0u, ctx->d_err);

@@ -683,6 +683,14 @@ mgv_status mgv_op_create_sink(mgv_ctx* ctx, const mgv_sink_desc* d, mgv_op** out
     s.pool = d->pool->dev;
     mgv_status st = dev_alloc(o, (void**)&s.cursor, sizeof(unsigned long long));
     if (st == MGV_OK) st = dev_alloc(o, (void**)&s.chain, sizeof(uint32_t) * maxc);
+    if (st == MGV_OK) {
+        cudaError_t e = cudaMallocHost(&o->sk_land, sizeof(SinkLanding) + sizeof(uint32_t) * (size_t)maxc);
+        if (e == cudaSuccess) e = cudaHostGetDevicePointer(reinterpret_cast<void**>(&o->sk_land_dev), o->sk_land, 0);
+        if (e != cudaSuccess) {
+            if (o->sk_land) cudaFreeHost(o->sk_land);
+            st = fail(MGV_ENOMEM, "pinned host allocation");
+        }
+    }
     if (st != MGV_OK) {
         for (void* p : o->allocs) cudaFree(p);
         delete o;
@@ -721,6 +729,7 @@ mgv_status mgv_op_destroy(mgv_op* o) {
         if (ev) cudaEventDestroy(ev);
     if (o->h_res) cudaFreeHost(o->h_res);
     if (o->hb_land) cudaFreeHost(o->hb_land);
+    if (o->sk_land) cudaFreeHost(o->sk_land);
     if (o->rb_scratch) cudaFree(o->rb_scratch);
     if (o->gb_land) cudaFreeHost(o->gb_land);
     for (void* p : o->allocs) cudaFree(p);
@@ -816,25 +825,14 @@ static void hash_build_info(Op* o, const unsigned long long* m) {
     o->unique = m[3] == 0;
 }
 
-// Reads back a terminal operator's result after its stream completed.
-static mgv_status op_finish(Op* o, cudaStream_t s) {
-    switch (o->kind) {
-        case OpKind::Sink: {
-            unsigned long long rows = 0;
-            MGV_CUDA_TRY(cudaMemcpyAsync(&rows, o->sink.cursor, sizeof(rows), cudaMemcpyDeviceToHost, s));
-            std::vector<uint32_t> chain(o->sink.max_chunks);
-            MGV_CUDA_TRY(cudaMemcpyAsync(chain.data(), o->sink.chain, sizeof(uint32_t) * chain.size(),
-                                         cudaMemcpyDeviceToHost, s));
-            MGV_CUDA_TRY(cudaStreamSynchronize(s));
-            o->sink_rows = rows;
-            o->sink_chain.clear();
-            for (uint32_t id : chain)
-                if (id < o->sink_pool->nbuffers) o->sink_chain.push_back(id);
-            break;
-        }
-        default: break;
-    }
-    return MGV_OK;
+// Waits for `s` and reads what a sink has gathered (o->sk_land): the rows, the
+// buffer chain and the error word, with one kernel and one wait instead of
+// three copies and two.  The error word is reported (and cleared) as the status.
+static mgv_status sink_gathered(Op* o, cudaStream_t s) {
+    MGV_CUDA_TRY(launch_sink_land(o->sink, o->sk_land_dev, s, o->ctx));
+    MGV_CUDA_TRY(cudaStreamSynchronize(s));
+    const uint32_t w[2] = {o->sk_land->err[0], o->sk_land->err[1]};
+    return report_device_error(o->ctx, w, s);
 }
 
 mgv_status mgv_op_close(mgv_op* o, void* stream) {
@@ -876,9 +874,12 @@ mgv_status mgv_op_close(mgv_op* o, void* stream) {
             if (st == MGV_OK) hash_build_info(o, o->hb_land->meta);
             return st;
         }
-        st = check_device(o->ctx, s);
-        mgv_status st2 = op_finish(o, s);
-        if (st == MGV_OK) st = st2;
+        st = sink_gathered(o, s);  // the remaining terminal: a sink
+        if (st == MGV_ECUDA) return st;
+        o->sink_rows = o->sk_land->rows;  // kept, with their buffers, after a reported device error too
+        o->sink_chain.clear();
+        for (uint32_t c = 0; c < o->sink.max_chunks; ++c)
+            if (o->sk_land->chain[c] < o->sink_pool->nbuffers) o->sink_chain.push_back(o->sk_land->chain[c]);
         return st;
     }
     if (o->kind == OpKind::Partition) {
@@ -995,18 +996,14 @@ mgv_status mgv_sink_drain(mgv_op* o, int32_t* const* dst_cols, uint32_t ncols, u
     // the previous drain's copies complete first: its buffers go back to the pool
     mgv_status st = sink_finish_drain(o);
     if (st != MGV_OK) return st;
-    st = check_device(o->ctx, s);  // waits for the consumes; a pool that ran dry is reported here
+    st = sink_gathered(o, s);  // waits for the consumes; a pool that ran dry is reported here
     if (st != MGV_OK) return st;
-    unsigned long long gathered = 0;
-    std::vector<uint32_t> chain(o->sink.max_chunks);
-    MGV_CUDA_TRY(cudaMemcpyAsync(&gathered, o->sink.cursor, sizeof(gathered), cudaMemcpyDeviceToHost, s));
-    MGV_CUDA_TRY(cudaMemcpyAsync(chain.data(), o->sink.chain, sizeof(uint32_t) * chain.size(), cudaMemcpyDeviceToHost,
-                                 s));
-    MGV_CUDA_TRY(cudaStreamSynchronize(s));
+    const unsigned long long gathered = o->sk_land->rows;
+    const uint32_t* chain = o->sk_land->chain;
     const uint64_t cap = o->sink.capacity;
     const uint64_t chunks = (gathered + cap - 1) / cap;
     std::vector<uint32_t> ids;
-    for (uint64_t c = 0; c < chunks && c < chain.size(); ++c) {
+    for (uint64_t c = 0; c < chunks && c < o->sink.max_chunks; ++c) {
         if (chain[c] >= o->sink_pool->nbuffers) return fail(MGV_EDEVICE, "sink chunk without a buffer");
         ids.push_back(chain[c]);
     }

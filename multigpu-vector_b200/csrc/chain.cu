@@ -166,6 +166,21 @@ __device__ __forceinline__ void sink_flush(const ChainDev& a, const SinkStage& s
     __syncwarp();  // the staging is free again
 }
 
+__global__ void k_sink_land(SinkView s, SinkLanding* land, const uint32_t* err) {
+    for (uint32_t c = threadIdx.x; c < s.max_chunks; c += blockDim.x) land->chain[c] = s.chain[c];
+    if (threadIdx.x == 0) {
+        land->err[0] = err[0];
+        land->err[1] = err[1];
+        land->rows = *s.cursor;
+    }
+}
+
+cudaError_t launch_sink_land(const SinkView& sv, SinkLanding* land, cudaStream_t s, Context* ctx) {
+    k_sink_land<<<1, 256, 0, s>>>(sv, land, ctx->d_err);
+    ctx->launches++;
+    return cudaGetLastError();
+}
+
 // ---- group tables ------------------------------------------------------------
 //
 // Both tables use Fibonacci hashing, (g * 2654435769) >> (32 - log2 cap), and
@@ -883,9 +898,8 @@ cudaError_t launch_cells(const ChainDev* d_scans, const BatchItem* items, uint32
     if (nitems == 0) return cudaSuccess;
     const size_t smem = kRingBytes + smem_cells_bytes(kCellSlots) + sizeof(int32_t) * kMaxCellRanges +
                         sizeof(uint16_t) * kCellLut;
-    cudaError_t e = cudaFuncSetAttribute(k_batch_cells, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-    const int grid = (int)std::min<uint64_t>((uint64_t)ctx->prop.multiProcessorCount, nitems);
+    const int grid =
+        (int)std::min<uint64_t>((uint64_t)occupancy_grid((const void*)k_batch_cells, kChainBlock, smem, ctx), nitems);
     k_batch_cells<<<grid, kChainBlock, smem, s>>>(d_scans, items, nitems, ctx->d_err);
     ctx->launches++;
     return cudaGetLastError();
@@ -905,11 +919,7 @@ cudaError_t launch_batch(const ChainDev* d_qs, const BatchItem* probe_items, uin
                          uint32_t item_order, cudaStream_t s, Context* ctx) {
     if (n_probe == 0) return cudaSuccess;
     const size_t smem = kRingBytes + smem_groups_bytes(kMaxSmemGroups);
-    cudaError_t e = cudaFuncSetAttribute(k_batch_probe, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-    int per_sm = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_batch_probe, kChainBlock, smem);
-    per_sm = std::max(per_sm, 1);
+    int per_sm = blocks_per_sm((const void*)k_batch_probe, kChainBlock, smem, ctx);
     if (ctas_per_sm > 0 && ctas_per_sm < per_sm) per_sm = ctas_per_sm;
     const int grid = (int)std::min<uint64_t>((uint64_t)per_sm * ctx->prop.multiProcessorCount, n_probe);
     k_batch_probe<<<grid, kChainBlock, smem, s>>>(d_qs, probe_items, n_probe, item_order, ctx->d_err);
@@ -924,10 +934,6 @@ static cudaError_t launch_chain_t(const ChainDev& d, uint64_t n, cudaStream_t s,
     const size_t smem = chain_ring_bytes<SEL, TERM>() + smem_groups_bytes(d.smem_groups) +
                         (TERM == kTermSink ? (kSinkBlock / 32) * sizeof(SinkStage) : 0);
     constexpr int block = chain_block<TERM>();
-    if (smem > 48 * 1024) {
-        cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return e;
-    }
     const int full = occupancy_grid((const void*)k, block, smem, ctx);
     // row offsets inside the kernel are 32-bit: launch at most 2^31 rows at a time
     constexpr uint64_t kChunk = 1ull << 31;

@@ -17,12 +17,22 @@ namespace mgv {
 
 constexpr int kBlock = 256;
 
-int occupancy_grid(const void* kernel, int block, size_t smem, const Context* ctx) {
+int blocks_per_sm(const void* kernel, int block, size_t smem, const Context* ctx) {
+    std::lock_guard<std::mutex> lk(ctx->fit_mu);
+    for (const Context::Fit& f : ctx->fits)
+        if (f.kernel == kernel && f.block == block && f.smem == smem) return f.per_sm;
+    cudaFuncAttributes fa;
+    if (cudaFuncGetAttributes(&fa, kernel) == cudaSuccess)
+        (void)cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   (int)(ctx->prop.sharedMemPerBlockOptin - fa.sharedSizeBytes));
     int per_sm = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, block, smem) != cudaSuccess ||
-        per_sm < 1)
-        per_sm = 1;
-    return per_sm * ctx->prop.multiProcessorCount;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, block, smem) != cudaSuccess || per_sm < 1) return 1;
+    ctx->fits.push_back(Context::Fit{kernel, block, smem, per_sm});
+    return per_sm;
+}
+
+int occupancy_grid(const void* kernel, int block, size_t smem, const Context* ctx) {
+    return blocks_per_sm(kernel, block, smem, ctx) * ctx->prop.multiProcessorCount;
 }
 
 static inline bool aligned32(const void* p) { return p == nullptr || ((uintptr_t)p & 31u) == 0; }

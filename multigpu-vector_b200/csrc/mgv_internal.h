@@ -123,6 +123,15 @@ struct Context {
     mgv_batch_config batch_tuned{};  // the batch autotuner's last choice
     bool has_batch_tuned = false;
     std::mutex mu;
+    // CTAs per SM of each launch shape used so far (blocks_per_sm)
+    struct Fit {
+        const void* kernel;
+        int block;
+        size_t smem;
+        int per_sm;
+    };
+    mutable std::mutex fit_mu;
+    mutable std::vector<Fit> fits;
 };
 
 enum class OpKind { Select, Aggregate, HashBuild, HashProbe, Sink, Groupby, Partition };
@@ -156,6 +165,8 @@ struct Op {
     SinkView sink{};
     uint64_t sink_rows = 0;
     std::vector<uint32_t> sink_chain;
+    struct SinkLanding* sk_land = nullptr;  // pinned, mapped: max_chunks ids
+    struct SinkLanding* sk_land_dev = nullptr;
     // delivery channel (mgv_sink_drain): copies run on their own stream; the
     // buffers of the copy in flight return to the pool when it completes
     cudaStream_t drain_stream = nullptr;
@@ -213,6 +224,11 @@ struct LaunchCfg {
     int block;
 };
 
+// CTAs of a launch shape that fit one SM (at least 1).  The first call for a
+// shape also raises the kernel's dynamic shared memory limit to what the
+// device allows; later ones are a look-up, where asking the runtime each time
+// took 2 to 3 us of a launch.
+int blocks_per_sm(const void* kernel, int block, size_t smem, const Context* ctx);
 int occupancy_grid(const void* kernel, int block, size_t smem, const Context* ctx);
 
 cudaError_t launch_fill_u64(unsigned long long* p, uint64_t n, unsigned long long v, cudaStream_t s,
@@ -296,6 +312,13 @@ struct ChainArgs {
     SinkView sink;
 };
 cudaError_t launch_chain(const ChainArgs& a, cudaStream_t s, Context* ctx);
+// What a sink has gathered, handed to the host by one kernel.
+struct SinkLanding {
+    uint32_t err[2];
+    unsigned long long rows;
+    uint32_t chain[1];  // max_chunks buffer ids
+};
+cudaError_t launch_sink_land(const SinkView& sv, SinkLanding* land, cudaStream_t s, Context* ctx);
 
 // Device-side parameters of one chain (one query of a batch).
 struct ChainDev {

@@ -193,10 +193,6 @@ cudaError_t launch_partition_scatter(const int32_t* const* cols, uint32_t ncols,
     for (uint32_t c = 0; c < ncols; ++c) in.cols[c] = cols[c];
     const size_t smem = part_scatter_smem(mask + 1);
     const void* k = has_sel ? (const void*)k_part_scatter<true> : (const void*)k_part_scatter<false>;
-    if (smem > 48 * 1024) {
-        cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return e;
-    }
     int grid = occupancy_grid(k, kPartBlock, smem, ctx);
     const uint64_t need = (n + kPartTile - 1) / kPartTile;
     if ((uint64_t)grid > need) grid = (int)need;

@@ -470,12 +470,7 @@ cudaError_t launch_v(const int32_t* keys, const int32_t* pays, uint64_t n, const
                         (size_t)3 * kConsumerWarps * queue_len<R>() * sizeof(int32_t) +
                         kConsumerWarps * sizeof(uint32_t) + 2 * S * sizeof(uint64_t);
     auto launch = [&](auto k, auto... extra) -> cudaError_t {
-        cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return e;
-        int per_sm = 0;
-        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, kThreads, smem);
-        if (e != cudaSuccess) return e;
-        if (per_sm < 1) per_sm = 1;
+        int per_sm = blocks_per_sm((const void*)k, kThreads, smem, ctx);
         if (ctas_per_sm > 0 && ctas_per_sm < per_sm) per_sm = ctas_per_sm;
         uint64_t grid = (uint64_t)per_sm * ctx->prop.multiProcessorCount;
         if (grid > cut.tiles) grid = cut.tiles ? cut.tiles : 1;

@@ -279,9 +279,21 @@ __host__ __device__ constexpr uint32_t tile_copies(uint32_t regions) {
     while (f < 32 && 2 * f * regions <= kTileCounters) f *= 2;
     return f;
 }
+// Shared memory for jobs of up to `regions` regions: a smaller job may use more
+// counters than the largest (200 regions x 4 copies, 128 x 8), but never more
+// than kTileCounters while it has copies at all.
+__host__ __device__ constexpr size_t tile_counter_bytes(uint32_t regions) {
+    return 4ull * (regions > kTileCounters ? regions : kTileCounters);
+}
+constexpr bool tile_counters_fit() {
+    for (uint32_t r = 1; r <= kTileRegions; ++r)
+        if (4ull * r * tile_copies(r) > tile_counter_bytes(r)) return false;
+    return true;
+}
+static_assert(tile_counters_fit(), "a job's counters fit the space of every launch it can be part of");
 template <bool KO>
 __host__ __device__ constexpr size_t tile_smem(uint32_t regions) {
-    return (KO ? 6ull : 10ull) * tile_size<KO>() + 4ull * regions * tile_copies(regions) + 4ull * regions;
+    return (KO ? 6ull : 10ull) * tile_size<KO>() + tile_counter_bytes(regions) + 4ull * regions;
 }
 template <bool KO>
 __device__ __forceinline__ TileSpace<KO> tile_space(unsigned char* base, uint32_t regions) {

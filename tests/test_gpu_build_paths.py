@@ -10,6 +10,7 @@ import pytest
 import mgv
 import pyoracle as po
 from gpu_util import dev
+from querymix import make_query_columns, oracle_answer
 
 pytestmark = pytest.mark.gpu
 INT32_MIN = -(1 << 31)
@@ -84,3 +85,21 @@ def test_build_more_regions_than_a_tile_sorts(ctx, torch_cuda):
     assert hb.result().rows == n and hb.result().has_duplicates == 0
     for o in (probe, agg, hb):
         o.destroy()
+
+
+def test_batch_tables_of_many_region_counts(ctx, torch_cuda):
+    """One launch over tables of 200, 128, 100, 64, 3, 1 and 0 regions (8192
+    rows each at load factor 0.5): the rank counters of a tile are replicated
+    more for a smaller table, so the largest one does not need the most."""
+    mix = []
+    for i, regions in enumerate([200, 128, 100, 64, 3, 1, 0]):
+        nb, npr = regions * 8192, 30011 + 1000 * i
+        cols = make_query_columns(ctx, torch_cuda, nb, npr, 100, 0x5EED0F51 + i)
+        mix.append(dict(nb=nb, npr=npr, bound=700, G=100, cols=cols))
+    b = mgv.Batch(ctx, [mgv.query_desc(q["cols"][0], q["nb"], *q["cols"][1:], q["npr"], q["bound"], q["G"])
+                        for q in mix], mgv.BatchConfig(0.5))
+    for _ in range(2):
+        b.run()
+    for i, q in enumerate(mix):
+        assert b.result(i) == oracle_answer(q), i
+    b.destroy()

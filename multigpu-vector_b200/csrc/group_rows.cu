@@ -163,8 +163,9 @@ __device__ unsigned long long* sort_pairs(unsigned long long* a, unsigned long l
 
 // The landing zone's header: the error word, then the groups found.
 __device__ __forceinline__ void land_header(GroupLanding* land, const uint32_t* err, uint32_t n) {
-    land->err[0] = err[0];
-    land->err[1] = err[1];
+    const uint32_t e0 = err[0], e1 = err[1];  // both reads before a write they might alias
+    land->err[0] = e0;
+    land->err[1] = e1;
     land->count = n;
 }
 

@@ -157,11 +157,14 @@ cudaError_t launch_select_agg(const int32_t* filt, int32_t bound, bool has_sel, 
 }
 
 __global__ void k_agg_land(unsigned long long* acc, unsigned long long* land, const uint32_t* err) {
-    if (threadIdx.x != 0) return;
-    land[0] = (unsigned long long)err[1] << 32 | err[0];
-    land[1] = acc[0];
-    land[2] = acc[1];
-    acc[0] = acc[1] = 0;
+    if (threadIdx.x > 2) return;  // a lane per word: the reads overlap (one lane, one word after the other: 0.4 to 1.4 us more)
+    if (threadIdx.x == 0) {
+        land[0] = (unsigned long long)err[1] << 32 | err[0];
+    } else {
+        unsigned long long* a = acc + threadIdx.x - 1;
+        land[threadIdx.x] = *a;
+        *a = 0;
+    }
 }
 
 cudaError_t launch_agg_land(unsigned long long* acc, unsigned long long* land, cudaStream_t s, Context* ctx) {

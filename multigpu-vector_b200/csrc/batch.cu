@@ -116,7 +116,8 @@ mgv_status enqueue_run(mgv_batch* b, cudaStream_t s) {
     layout.t.key_only = b->key_only;
     layout.shift = kRegionShift;
     MGV_CUDA_TRY(launch_build_regions(b->d_jobs, layout, (uint32_t)b->q.size(), b->d_build_items, b->n_build, 0,
-                                      b->total_regions, b->max_job_regions, b->rsc, false, true, nullptr, s, ctx));
+                                      b->total_regions, b->max_job_regions, b->rsc, false, true, nullptr, false, s,
+                                      ctx));
     MGV_CUDA_TRY(launch_batch(b->d_qs, b->d_probe_items, b->n_probe, (int)b->cfg.probe_ctas_per_sm, b->cfg.item_order,
                               s, ctx));
     MGV_CUDA_TRY(launch_batch_compact(b->d_outs, b->d_compact_items, b->n_compact, s, ctx));

@@ -1185,8 +1185,8 @@ static mgv_status consume_cols(Op* head, const int32_t* const* cols, uint32_t nc
                 term->hb_landed = true;
                 return MGV_OK;
             }
-            if (fresh) MGV_CUDA_TRY(cudaMemsetAsync(t.meta, 0, 4 * sizeof(unsigned long long), s));
             if (n < kRegionBuildMinRows || n >= (1ull << 31) || table_regions(t) > kMaxRegionsPerJob) {
+                if (fresh) MGV_CUDA_TRY(cudaMemsetAsync(t.meta, 0, 4 * sizeof(unsigned long long), s));
                 if (fresh) MGV_CUDA_TRY(launch_fill_u64(t.slots, 4ull * t.nbuckets, kEmptySlot, s, ctx));
                 MGV_CUDA_TRY(launch_build(cols[kc], pays, filt, bound, sel != nullptr, n, t, s, ctx));
                 return MGV_OK;
@@ -1212,15 +1212,21 @@ static mgv_status consume_cols(Op* head, const int32_t* const* cols, uint32_t nc
                     term->rb_scratch = nullptr;
                     term->rb_bytes = 0;
                 }
+                term->rb_zeroed = 0;
                 MGV_CUDA_TRY(cudaMalloc(&term->rb_scratch, need));
                 term->rb_bytes = need;
             }
             const RegionScratch sc = carve_region_scratch(term->rb_scratch, job.nregions, staged, n);
+            const bool captured = !skip_reset(true, s);  // a capture runs nothing now: it leaves the scratch as it is
+            const bool zeroed = !captured && term->rb_zeroed == job.nregions;
+            term->rb_zeroed = 0;  // until every launch is made
             if (part_run)
-                MGV_CUDA_TRY(launch_build_regions_partitioned(job, term->hb_part_ends, n, sc, term->hb_land_dev, s, ctx));
+                MGV_CUDA_TRY(launch_build_regions_partitioned(job, term->hb_part_ends, n, sc, term->hb_land_dev, zeroed, s,
+                                                              ctx));
             else
                 MGV_CUDA_TRY(launch_build_regions(nullptr, job, 1, nullptr, 0, n, job.nregions, job.nregions, sc, exact,
-                                                  fresh, term->hb_land_dev, s, ctx));
+                                                  fresh, term->hb_land_dev, zeroed, s, ctx));
+            if (!captured) term->rb_zeroed = job.nregions;
             term->hb_landed = true;
             return MGV_OK;
         }

@@ -213,6 +213,7 @@ struct Op {
     // shared-memory build scratch (hash_build), grown on demand
     void* rb_scratch = nullptr;
     size_t rb_bytes = 0;
+    uint32_t rb_zeroed = 0;  // regions for which the scratch was left zeroed (0: none)
     // device allocations owned by this op
     std::vector<void*> allocs;
 };
@@ -379,8 +380,11 @@ struct RegionJob {
     uint32_t pad;
 };
 struct RegionScratch {
-    uint32_t* cursor;         // [regions] rows placed, zeroed together with ctl (region_zero_bytes)
+    // cursor, ctl and meta are zeroed together (region_zero_bytes), before a
+    // launch and, where the launch lands one table's counters, again by its end
+    uint32_t* cursor;         // [regions] rows placed
     uint32_t* ctl;            // [2] rows left for the global insert, CTAs done
+    unsigned long long* meta; // [4] the counters of a fresh table while it is built (TableView::meta)
     uint32_t* hist;           // [regions] rows per region (exact ranges)
     uint32_t* start;          // [regions + 1] first staging row of each region (exact ranges)
     unsigned long long* staging;  // {key, payload}, region-major
@@ -405,18 +409,20 @@ cudaError_t region_build_init();  // once per device: the kernels' shared memory
 // job0.  exact: staging ranges from a histogram (the jobs' stage0 and cap are
 // not used).  fresh: the tables hold nothing yet and are not cleared
 // beforehand; every region is written.  land: nullable, where one table's
-// counters go afterwards.
+// counters go afterwards; a fresh table's own need no clearing then.  zeroed:
+// the scratch is as the last such launch over as many regions left it.
 cudaError_t launch_build_regions(const RegionJob* d_jobs, const RegionJob& job0, uint32_t njobs,
                                  const struct BatchItem* items, uint32_t nitems, uint64_t n, uint32_t total_regions,
                                  uint32_t max_job_regions, const RegionScratch& sc, bool exact, bool fresh,
-                                 TableLanding* land, cudaStream_t s, Context* ctx);
+                                 TableLanding* land, bool zeroed, cudaStream_t s, Context* ctx);
 // A fresh radix-laid-out table built from a partition op's single run on its
 // radix bits (ends[p] = one past partition p's last row): per-partition
 // staging in the partition's own range, then the region build.  Only when
 // every partition slice is whole regions (region_build_partitioned_fits).
 bool region_build_partitioned_fits(const TableView& t);
 cudaError_t launch_build_regions_partitioned(const RegionJob& job, const unsigned long long* ends, uint64_t n,
-                                             const RegionScratch& sc, TableLanding* land, cudaStream_t s, Context* ctx);
+                                             const RegionScratch& sc, TableLanding* land, bool zeroed, cudaStream_t s,
+                                             Context* ctx);
 // A fresh table of at most kRegionBuckets buckets from all its rows.
 cudaError_t launch_build_small(const RegionJob& job, uint32_t n, TableLanding* land, cudaStream_t s, Context* ctx);
 cudaError_t launch_table_land(const TableView& t, TableLanding* land, cudaStream_t s, Context* ctx);

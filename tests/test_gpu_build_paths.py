@@ -73,6 +73,50 @@ def test_build_paths(ctx, torch_cuda, n, lf, kind, payload):
         o.destroy()
 
 
+@pytest.mark.parametrize("radix_bits", [0, 4])
+def test_build_scratch_across_a_capture(ctx, torch_cuda, radix_bits):
+    """A build leaves its scratch zeroed for the next one; a captured build,
+    which runs when it is replayed, neither relies on that nor claims it."""
+    torch, n = torch_cuda, 150_001
+    sides = [(po.gen_perm(n, 0x5EED0F61 + i), po.gen_uniform(n, 0x5EED0F61 + i, 1, 0, 1 << 20)) for i in range(2)]
+    sides[1][0][::1000] = INT32_MIN
+    pk, pp = po.gen_uniform(20011, 0x5EED0F63, 0, 0, n + n // 8), po.gen_uniform(20011, 0x5EED0F63, 1, 0, 1 << 20)
+    cols = [[dev(torch, c) for c in side] for side in sides]
+    probe_cols = [dev(torch, pk), dev(torch, pp)]
+    hb = mgv.Op.hash_build(ctx, 0, 1, n, 0.5, radix_bits=radix_bits)
+    agg = mgv.Op.aggregate(ctx, 1, 2)
+    probe = mgv.Op.hash_probe(ctx, 0, hb, agg)
+
+    def check(side):
+        probe.open(); probe.consume_columns(probe_cols, len(pk)); probe.close()
+        assert agg.result() == po.Chain(*side).probe_agg(pk, pp)
+        assert hb.result().reserved_key_rows == int((side[0] == INT32_MIN).sum())
+
+    def build(i):
+        hb.open(); hb.consume_columns(cols[i], n); hb.close()
+        check(sides[i])
+
+    build(0)
+    build(1)
+    st, g = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+    torch.cuda.synchronize()
+    with torch.cuda.graph(g, stream=st):
+        hb.open(stream=st.cuda_stream)
+        hb.consume_columns(cols[1], n, stream=st.cuda_stream)
+    with torch.cuda.stream(st):
+        g.replay()
+    hb.close(stream=st.cuda_stream)
+    check(sides[1])
+    build(0)
+    with torch.cuda.stream(st):
+        g.replay()
+    torch.cuda.synchronize()
+    build(0)
+    build(1)
+    for o in (probe, agg, hb):
+        o.destroy()
+
+
 def test_build_more_regions_than_a_tile_sorts(ctx, torch_cuda):
     """2^23 {key, payload} rows at load factor 0.2: 5120 regions."""
     n = 1 << 23

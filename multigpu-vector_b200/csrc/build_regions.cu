@@ -107,7 +107,7 @@ struct StageOut {
 __device__ __forceinline__ void overflow_put(const StageOut& o, unsigned long long v, uint32_t job) {
     const uint32_t i = atomicAdd(o.ctl, 1u);
     o.ovf[i] = v;
-    o.ovf_job[i] = job;
+    if (o.ovf_job) o.ovf_job[i] = job;
 }
 
 // Row `i` of a region (counted from the region's first) into its range.
@@ -981,13 +981,13 @@ static size_t align_scratch(size_t x) { return (x + 255) & ~(size_t)255; }
 
 size_t region_zero_bytes(uint32_t regions) { return align_scratch(4ull * regions) + 8 + 32; }
 
-size_t region_scratch_bytes(uint32_t regions, uint64_t staged, uint64_t rows) {
+size_t region_scratch_bytes(uint32_t regions, uint64_t staged, uint64_t rows, bool one_job) {
     auto a = align_scratch;
     return a(region_zero_bytes(regions)) + a(4ull * regions) + a(4ull * (regions + 1)) + a(8ull * staged) + a(8ull * rows) +
-           a(4ull * rows);
+           (one_job ? 0 : a(4ull * rows));
 }
 
-RegionScratch carve_region_scratch(void* base, uint32_t regions, uint64_t staged, uint64_t rows) {
+RegionScratch carve_region_scratch(void* base, uint32_t regions, uint64_t staged, uint64_t rows, bool one_job) {
     auto a = align_scratch;
     unsigned char* p = static_cast<unsigned char*>(base);
     RegionScratch s;
@@ -1003,7 +1003,7 @@ RegionScratch carve_region_scratch(void* base, uint32_t regions, uint64_t staged
     p += a(8ull * staged);
     s.ovf = reinterpret_cast<unsigned long long*>(p);
     p += a(8ull * rows);
-    s.ovf_job = reinterpret_cast<uint32_t*>(p);
+    s.ovf_job = one_job ? nullptr : reinterpret_cast<uint32_t*>(p);
     return s;
 }
 

@@ -1194,17 +1194,18 @@ static mgv_status consume_cols(Op* head, const int32_t* const* cols, uint32_t nc
             // the hash spreads an unpartitioned table's rows evenly: fixed staging shares,
             // and regions small enough for two per SM; a radix layout follows the raw
             // key bits: exact staging ranges
-            const bool exact = t.radix_mask != 0;
+            bool exact = t.radix_mask != 0 || term->rb_exact;
+            const bool radix = t.radix_mask != 0;
             const bool part_run = fresh && term->hb_part_ends && !sel && region_build_partitioned_fits(t);
-            if (!exact)
+            if (!radix)
                 while (job.shift > kMinRegionShift &&
                        (t.nbuckets >> job.shift) < 2u * (uint32_t)ctx->prop.multiProcessorCount)
                     --job.shift;
             job.nregions = (t.nbuckets + (1u << job.shift) - 1) >> job.shift;
             job.cap = region_share(n, job.nregions, t, job.shift);
-            const uint64_t staged = exact ? n : (uint64_t)job.nregions * job.cap;
+            uint64_t staged = exact ? n : (uint64_t)job.nregions * job.cap;
             // the scratch is kept by the operator and grown on demand
-            const size_t need = region_scratch_bytes(job.nregions, staged, n);
+            size_t need = region_scratch_bytes(job.nregions, staged, n, true);
             if (term->rb_bytes < need) {
                 if (term->rb_scratch) {
                     MGV_CUDA_TRY(cudaStreamSynchronize(s));
@@ -1213,10 +1214,20 @@ static mgv_status consume_cols(Op* head, const int32_t* const* cols, uint32_t nc
                     term->rb_bytes = 0;
                 }
                 term->rb_zeroed = 0;
-                MGV_CUDA_TRY(cudaMalloc(&term->rb_scratch, need));
+                cudaError_t e = cudaMalloc(&term->rb_scratch, need);
+                if (e == cudaErrorMemoryAllocation && !exact) {
+                    // the shares take up to 24 bytes a row, exact ranges 16
+                    (void)cudaGetLastError();
+                    term->rb_exact = exact = true;
+                    staged = n;
+                    need = region_scratch_bytes(job.nregions, staged, n, true);
+                    e = cudaMalloc(&term->rb_scratch, need);
+                }
+                if (e != cudaSuccess) term->rb_scratch = nullptr;
+                MGV_CUDA_TRY(e);
                 term->rb_bytes = need;
             }
-            const RegionScratch sc = carve_region_scratch(term->rb_scratch, job.nregions, staged, n);
+            const RegionScratch sc = carve_region_scratch(term->rb_scratch, job.nregions, staged, n, true);
             const bool captured = !skip_reset(true, s);  // a capture runs nothing now: it leaves the scratch as it is
             const bool zeroed = !captured && term->rb_zeroed == job.nregions;
             term->rb_zeroed = 0;  // until every launch is made

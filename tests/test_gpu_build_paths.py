@@ -117,6 +117,34 @@ def test_build_scratch_across_a_capture(ctx, torch_cuda, radix_bits):
         o.destroy()
 
 
+def test_build_without_room_for_staging_shares(ctx, torch_cuda):
+    """With room for exact staging ranges (16 bytes a row) but not for shares
+    of twice the expected rows (24), the build takes the exact ranges."""
+    torch, n = torch_cuda, 1 << 24
+    bk, bp = po.gen_perm(n, 0x5EED0F71), po.gen_uniform(n, 0x5EED0F71, 1, 0, 1 << 20)
+    pk, pp = po.gen_uniform(50021, 0x5EED0F72, 0, 0, n + n // 8), po.gen_uniform(50021, 0x5EED0F72, 1, 0, 1 << 20)
+    cols, probe_cols = [dev(torch, bk), dev(torch, bp)], [dev(torch, pk), dev(torch, pp)]
+    hb = mgv.Op.hash_build(ctx, 0, 1, n, 0.5)
+    agg = mgv.Op.aggregate(ctx, 1, 2)
+    probe = mgv.Op.hash_probe(ctx, 0, hb, agg)
+    torch.cuda.empty_cache()
+    hog = torch.empty(torch.cuda.mem_get_info()[0] - 20 * n, dtype=torch.uint8, device="cuda")
+    hb.open()
+    l0 = ctx.launches
+    hb.consume_columns(cols, n)
+    assert ctx.launches - l0 == 5  # histogram, scan, staging, regions, global insert
+    hb.close()
+    del hog
+    torch.cuda.empty_cache()
+    for _ in range(2):
+        probe.open(); probe.consume_columns(probe_cols, len(pk)); probe.close()
+        assert agg.result() == po.Chain(bk, bp).probe_agg(pk, pp)
+        assert hb.result().rows == n and hb.result().has_duplicates == 0
+        hb.open(); hb.consume_columns(cols, n); hb.close()
+    for o in (probe, agg, hb):
+        o.destroy()
+
+
 def test_build_more_regions_than_a_tile_sorts(ctx, torch_cuda):
     """2^23 {key, payload} rows at load factor 0.2: 5120 regions."""
     n = 1 << 23

@@ -238,7 +238,7 @@ mgv_status create_batch(mgv_ctx* ctx, const mgv_query_desc* qs, uint32_t nq, con
         delete b;
         return fail(MGV_EUNSUPPORTED, "a batch holds fewer than 2^31 build rows");
     }
-    const size_t rsc_off = take(region_scratch_bytes(total_regions, staged, build_total, false));
+    const size_t rsc_off = take(region_scratch_bytes(total_regions, staged, build_total, false, b->key_only != 0));
     const size_t outs_off = take(sizeof(BatchOut) * std::max(nq, 1u));
     b->ordered.assign(nq, 0);
     std::vector<uint32_t> sorts;
@@ -295,7 +295,7 @@ mgv_status create_batch(mgv_ctx* ctx, const mgv_query_desc* qs, uint32_t nq, con
     b->out_counts = reinterpret_cast<uint32_t*>(A + counts_off);
     b->d_qs = reinterpret_cast<ChainDev*>(A + qs_off);
     b->d_jobs = reinterpret_cast<RegionJob*>(A + jobs_off);
-    b->rsc = carve_region_scratch(A + rsc_off, total_regions, staged, build_total, false);
+    b->rsc = carve_region_scratch(A + rsc_off, total_regions, staged, build_total, false, b->key_only != 0);
     b->total_regions = total_regions;
     b->max_job_regions = max_job_regions;
     b->d_outs = reinterpret_cast<BatchOut*>(A + outs_off);

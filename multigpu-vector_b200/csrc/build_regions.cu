@@ -981,13 +981,15 @@ static size_t align_scratch(size_t x) { return (x + 255) & ~(size_t)255; }
 
 size_t region_zero_bytes(uint32_t regions) { return align_scratch(4ull * regions) + 8 + 32; }
 
-size_t region_scratch_bytes(uint32_t regions, uint64_t staged, uint64_t rows, bool one_job) {
+size_t region_scratch_bytes(uint32_t regions, uint64_t staged, uint64_t rows, bool one_job, bool key_only) {
     auto a = align_scratch;
-    return a(region_zero_bytes(regions)) + a(4ull * regions) + a(4ull * (regions + 1)) + a(8ull * staged) + a(8ull * rows) +
+    return a(region_zero_bytes(regions)) + a(4ull * regions) + a(4ull * (regions + 1)) +
+           a((key_only ? 4ull : 8ull) * staged) + a(8ull * rows) +
            (one_job ? 0 : a(4ull * rows));
 }
 
-RegionScratch carve_region_scratch(void* base, uint32_t regions, uint64_t staged, uint64_t rows, bool one_job) {
+RegionScratch carve_region_scratch(void* base, uint32_t regions, uint64_t staged, uint64_t rows, bool one_job,
+                                   bool key_only) {
     auto a = align_scratch;
     unsigned char* p = static_cast<unsigned char*>(base);
     RegionScratch s;
@@ -1000,7 +1002,7 @@ RegionScratch carve_region_scratch(void* base, uint32_t regions, uint64_t staged
     s.start = reinterpret_cast<uint32_t*>(p);
     p += a(4ull * (regions + 1));
     s.staging = reinterpret_cast<unsigned long long*>(p);
-    p += a(8ull * staged);
+    p += a((key_only ? 4ull : 8ull) * staged);
     s.ovf = reinterpret_cast<unsigned long long*>(p);
     p += a(8ull * rows);
     s.ovf_job = one_job ? nullptr : reinterpret_cast<uint32_t*>(p);

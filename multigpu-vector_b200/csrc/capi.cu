@@ -1205,7 +1205,7 @@ static mgv_status consume_cols(Op* head, const int32_t* const* cols, uint32_t nc
             job.cap = region_share(n, job.nregions, t, job.shift);
             uint64_t staged = exact ? n : (uint64_t)job.nregions * job.cap;
             // the scratch is kept by the operator and grown on demand
-            size_t need = region_scratch_bytes(job.nregions, staged, n, true);
+            size_t need = region_scratch_bytes(job.nregions, staged, n, true, t.key_only != 0);
             if (term->rb_bytes < need) {
                 if (term->rb_scratch) {
                     MGV_CUDA_TRY(cudaStreamSynchronize(s));
@@ -1216,18 +1216,18 @@ static mgv_status consume_cols(Op* head, const int32_t* const* cols, uint32_t nc
                 term->rb_zeroed = 0;
                 cudaError_t e = cudaMalloc(&term->rb_scratch, need);
                 if (e == cudaErrorMemoryAllocation && !exact) {
-                    // the shares take up to 24 bytes a row, exact ranges 16
+                    // the shares take up to 24 bytes a row, exact ranges 16 (key-only: 16, 12)
                     (void)cudaGetLastError();
                     term->rb_exact = exact = true;
                     staged = n;
-                    need = region_scratch_bytes(job.nregions, staged, n, true);
+                    need = region_scratch_bytes(job.nregions, staged, n, true, t.key_only != 0);
                     e = cudaMalloc(&term->rb_scratch, need);
                 }
                 if (e != cudaSuccess) term->rb_scratch = nullptr;
                 MGV_CUDA_TRY(e);
                 term->rb_bytes = need;
             }
-            const RegionScratch sc = carve_region_scratch(term->rb_scratch, job.nregions, staged, n, true);
+            const RegionScratch sc = carve_region_scratch(term->rb_scratch, job.nregions, staged, n, true, t.key_only != 0);
             const bool captured = !skip_reset(true, s);  // a capture runs nothing now: it leaves the scratch as it is
             const bool zeroed = !captured && term->rb_zeroed == job.nregions;
             term->rb_zeroed = 0;  // until every launch is made

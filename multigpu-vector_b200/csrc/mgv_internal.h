@@ -401,8 +401,9 @@ struct TableLanding {
 void sort_group_rows(std::vector<mgv_group_row>& v);
 inline uint32_t table_regions(const TableView& t) { return (t.nbuckets + kRegionBuckets - 1) / kRegionBuckets; }
 size_t region_zero_bytes(uint32_t regions);
-size_t region_scratch_bytes(uint32_t regions, uint64_t staged, uint64_t rows, bool one_job);
-RegionScratch carve_region_scratch(void* base, uint32_t regions, uint64_t staged, uint64_t rows, bool one_job);
+size_t region_scratch_bytes(uint32_t regions, uint64_t staged, uint64_t rows, bool one_job, bool key_only);
+RegionScratch carve_region_scratch(void* base, uint32_t regions, uint64_t staged, uint64_t rows, bool one_job,
+                                   bool key_only);
 // Staging rows of each region when the ranges are fixed shares.
 uint32_t region_share(uint64_t rows, uint32_t nregions, const TableView& t, uint32_t shift);
 cudaError_t region_build_init();  // once per device: the kernels' shared memory limits

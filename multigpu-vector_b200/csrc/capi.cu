@@ -737,23 +737,31 @@ mgv_status mgv_op_destroy(mgv_op* o) {
     return MGV_OK;
 }
 
-// Whether an open on `s` may leave out the reset of what the last close left
-// clean: not while a graph is captured, whose replays need it every time.
-static bool skip_reset(bool clean, cudaStream_t s) {
-    if (!clean) return false;
+// Whether work on `s` is captured into a graph (where the runtime cannot say, it is taken to be).
+static bool capturing(cudaStream_t s) {
     cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(s, &st) != cudaSuccess) {
         (void)cudaGetLastError();
-        return false;
+        return true;
     }
-    return st == cudaStreamCaptureStatusNone;
+    return st != cudaStreamCaptureStatusNone;
+}
+
+// Before an open or a consume puts work of `o` on `s`.  Once a graph holds some
+// of it, a replay changes the device state at any time without the host taking
+// part: from then on no flag of the host says what that state is.
+static bool note_capture(Op* o, cudaStream_t s) {
+    const bool c = capturing(s);
+    if (c) o->graphed = true;
+    return c;
 }
 
 // Resets one operator's device state (at_open).
 static mgv_status op_reset(Op* o, cudaStream_t s) {
     switch (o->kind) {
         case OpKind::Aggregate:
-            if (!skip_reset(o->agg_clean, s))
+            note_capture(o, s);
+            if (o->graphed || !o->agg_clean)
                 MGV_CUDA_TRY(cudaMemsetAsync(o->d_acc, 0, 2 * sizeof(unsigned long long), s));
             o->agg_clean = true;  // until a consume or a close touches it
             o->agg_result = mgv_agg_result{0, 0};
@@ -779,7 +787,9 @@ static mgv_status op_reset(Op* o, cudaStream_t s) {
                 return fail(MGV_ESTATE, "hash_probe opened before its build side was closed");
             break;
         case OpKind::Groupby:
-            if (!skip_reset(o->gb_clean, s)) MGV_CUDA_TRY(launch_group_reset(o->gtab, o->gb_dev_count, s, o->ctx));
+            note_capture(o, s);
+            if (o->graphed || !o->gb_clean)
+                MGV_CUDA_TRY(launch_group_reset(o->gtab, o->gb_dev_count, s, o->ctx));
             o->gb_clean = true;  // until a consume or a close touches it
             o->gb_view = nullptr;
             o->gb_n = 0;
@@ -1108,6 +1118,7 @@ static mgv_status consume_cols(Op* head, const int32_t* const* cols, uint32_t nc
             const int32_t ca = term->agg.sum_col_a, cb = term->agg.sum_col_b;
             if (!ref_ok(ca) || !ref_ok(cb)) return fail(MGV_EINVAL, "aggregate column not in input");
             if (n == 0) return MGV_OK;
+            note_capture(term, s);
             term->agg_clean = false;
             // select -> aggregate: the masked fold, unless the context asks
             // for the warp-ballot compaction of the chain kernel
@@ -1144,6 +1155,7 @@ static mgv_status consume_cols(Op* head, const int32_t* const* cols, uint32_t nc
             const int32_t g = (int32_t)term->gb.group_col, v = term->gb.value_col;
             if (!ref_ok(g) || g == -1 || !ref_ok(v)) return fail(MGV_EINVAL, "group-by column not in input");
             if (n == 0) return MGV_OK;
+            note_capture(term, s);
             term->gb_clean = false;
             a.term = kTermGroupby;
             a.ref[0] = g;
@@ -1228,7 +1240,7 @@ static mgv_status consume_cols(Op* head, const int32_t* const* cols, uint32_t nc
                 term->rb_bytes = need;
             }
             const RegionScratch sc = carve_region_scratch(term->rb_scratch, job.nregions, staged, n, true, t.key_only != 0);
-            const bool captured = !skip_reset(true, s);  // a capture runs nothing now: it leaves the scratch as it is
+            const bool captured = capturing(s);  // a capture runs nothing now: it leaves the scratch as it is
             const bool zeroed = !captured && term->rb_zeroed == job.nregions;
             term->rb_zeroed = 0;  // until every launch is made
             if (part_run)

@@ -142,6 +142,7 @@ struct Op {
     Context* ctx = nullptr;
     Op* parent = nullptr;
     OpState state = OpState::Created;
+    bool graphed = false;  // an open or a consume of it was captured into a graph (for good)
     // select
     mgv_select_desc sel{};
     // aggregate

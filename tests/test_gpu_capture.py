@@ -1,0 +1,86 @@
+"""Operators whose open and consume were captured into a CUDA graph, replayed
+before and after a close, and then opened, fed and closed in the ordinary way:
+an open starts from nothing whatever a replay left on the device."""
+import pytest
+
+import mgv
+import pyoracle as po
+from gpu_util import dev
+
+pytestmark = pytest.mark.gpu
+
+
+def capture(torch, head, cols, n):
+    """A graph of one open and one consume on a stream of its own; the operator is left open."""
+    st, g = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+    torch.cuda.synchronize()
+    with torch.cuda.graph(g, stream=st):
+        head.open(stream=st.cuda_stream)
+        head.consume_columns(cols, n, stream=st.cuda_stream)
+
+    def replay():
+        with torch.cuda.stream(st):
+            g.replay()
+
+    return st, replay
+
+
+def result_chains(ctx, torch, n):
+    """name -> (head, its columns, terminal, other columns): select -> aggregate, probe -> aggregate, select ->
+    group-by of tables closed by one CTA and by many."""
+    nb = 3000
+    hb = mgv.Op.hash_build(ctx, 0, 1, nb)
+    bk, bp = po.gen_perm(nb, 0x5EED1101), po.gen_uniform(nb, 0x5EED1101, 1, 0, 1 << 20)
+    hb.open(); hb.consume_columns([dev(torch, bk), dev(torch, bp)], nb); hb.close()
+    agg, pagg = mgv.Op.aggregate(ctx, 0, -1), mgv.Op.aggregate(ctx, 1, 2)
+    small, large = mgv.Op.groupby(ctx, 0, 1, 1000), mgv.Op.groupby(ctx, 0, 1, 5000)
+    heads = {"select_agg": (mgv.Op.select(ctx, 1, 499, agg), agg),
+             "probe_agg": (mgv.Op.hash_probe(ctx, 0, hb, pagg), pagg),
+             "group_small": (mgv.Op.select(ctx, 1, 499, small), small),
+             "group_large": (mgv.Op.select(ctx, 1, 499, large), large)}
+    sides = [[po.gen_uniform(n, 0x5EED1102 + i, 0, 0, 1000), po.gen_uniform(n, 0x5EED1102 + i, 1, 0, 1000)]
+             for i in range(2)]
+    return heads, [[dev(torch, c) for c in s] for s in sides], hb
+
+
+@pytest.mark.parametrize("chain", ["select_agg", "probe_agg", "group_small", "group_large"])
+@pytest.mark.parametrize("open_captured", [True, False])
+def test_plain_pass_after_a_replay(ctx, torch_cuda, chain, open_captured):
+    torch, n = torch_cuda, 60_007
+    heads, sides, hb = result_chains(ctx, torch, n)
+    head, term = heads[chain]
+
+    def plain(i):
+        head.open(); head.consume_columns(sides[i], n); head.close()
+        return term.result()
+
+    want = [plain(0), plain(1)]
+    assert want[0] != want[1]
+    if open_captured:
+        st, replay = capture(torch, head, sides[1], n)
+    else:  # the consume alone
+        head.open()
+        st, g = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+        torch.cuda.synchronize()
+        with torch.cuda.graph(g, stream=st):
+            head.consume_columns(sides[1], n, stream=st.cuda_stream)
+
+        def replay():
+            with torch.cuda.stream(st):
+                g.replay()
+    replay()
+    head.close(stream=st.cuda_stream)
+    assert term.result() == want[1]
+    replay()
+    torch.cuda.synchronize()
+    assert plain(0) == want[0]
+    replay()
+    replay()
+    torch.cuda.synchronize()
+    assert plain(1) == want[1]
+    assert plain(0) == want[0]
+    head.open(); head.close()
+    assert term.result() in ((0, 0), [])
+    for h, t in heads.values():
+        h.destroy(); t.destroy()
+    hb.destroy()

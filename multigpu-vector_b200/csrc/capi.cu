@@ -877,7 +877,8 @@ mgv_status mgv_op_close(mgv_op* o, void* stream) {
         }
         if (o->kind == OpKind::Groupby) return close_groupby(o, s);
         if (o->kind == OpKind::HashBuild) {  // the error word and the table's counters, with one wait
-            if (!o->hb_landed) MGV_CUDA_TRY(launch_table_land(o->table, o->hb_land_dev, s, o->ctx));
+            // of a table that a graph holds, the last writer may be a replay that lands nothing
+            if (!o->hb_landed || o->graphed) MGV_CUDA_TRY(launch_table_land(o->table, o->hb_land_dev, s, o->ctx));
             MGV_CUDA_TRY(cudaStreamSynchronize(s));
             const uint32_t w[2] = {o->hb_land->err[0], o->hb_land->err[1]};
             st = report_device_error(o->ctx, w, s);
@@ -1189,6 +1190,7 @@ static mgv_status consume_cols(Op* head, const int32_t* const* cols, uint32_t nc
             const bool fresh = term->hb_fresh;
             term->hb_fresh = false;
             term->hb_landed = false;
+            const bool captured = note_capture(term, s);
             RegionJob job{t, cols[kc], pays, filt, bound, 0, 1, kRegionShift, 0, 0, 0};
             // a table of one region and few rows: one CTA reads them in a few
             // microseconds, less than a second launch costs
@@ -1240,7 +1242,7 @@ static mgv_status consume_cols(Op* head, const int32_t* const* cols, uint32_t nc
                 term->rb_bytes = need;
             }
             const RegionScratch sc = carve_region_scratch(term->rb_scratch, job.nregions, staged, n, true, t.key_only != 0);
-            const bool captured = capturing(s);  // a capture runs nothing now: it leaves the scratch as it is
+            // a capture runs nothing now: it leaves the scratch as it is
             const bool zeroed = !captured && term->rb_zeroed == job.nregions;
             term->rb_zeroed = 0;  // until every launch is made
             if (part_run)

@@ -84,3 +84,46 @@ def test_plain_pass_after_a_replay(ctx, torch_cuda, chain, open_captured):
     for h, t in heads.values():
         h.destroy(); t.destroy()
     hb.destroy()
+
+
+@pytest.mark.parametrize("radix_bits", [0, 4])
+@pytest.mark.parametrize("captured_rows,plain_rows", [(30_000, 150_001), (150_001, 30_000), (3_000, 150_001)])
+def test_replayed_build_is_closed_by_its_own_counters(ctx, torch_cuda, captured_rows, plain_rows, radix_bits):
+    """A graph of one build replayed over the rows of another, by any of the build paths: the close reads the
+    counters of the table as it is, whichever of them wrote it last."""
+    torch = torch_cuda
+    pk, pp = po.gen_uniform(20011, 0x5EED1112, 0, 0, 1 << 17), po.gen_uniform(20011, 0x5EED1112, 1, 0, 1 << 20)
+    probe_cols = [dev(torch, pk), dev(torch, pp)]
+    sides = []
+    for i, n in enumerate((captured_rows, plain_rows)):
+        keys = po.gen_perm(n, 0x5EED1113 + i) if i else po.gen_uniform(n, 0x5EED1113, 0, 0, n // 2)  # captured: repeated
+        sides.append((keys, po.gen_uniform(n, 0x5EED1113 + i, 1, 0, 1 << 20)))
+    cols = [[dev(torch, c) for c in side] for side in sides]
+    hb = mgv.Op.hash_build(ctx, 0, 1, max(captured_rows, plain_rows), radix_bits=radix_bits)
+    agg = mgv.Op.aggregate(ctx, 1, 2)
+    probe = mgv.Op.hash_probe(ctx, 0, hb, agg)
+
+    def check(i):
+        assert hb.result().rows == len(sides[i][0])
+        assert hb.result().has_duplicates == (1 - i)
+        probe.open(); probe.consume_columns(probe_cols, len(pk)); probe.close()
+        assert agg.result() == po.Chain(*sides[i]).probe_agg(pk, pp)
+
+    def build(i):
+        hb.open(); hb.consume_columns(cols[i], len(sides[i][0])); hb.close()
+        check(i)
+
+    build(0)
+    build(1)
+    st, replay = capture(torch, hb, cols[0], captured_rows)
+    replay()
+    hb.close(stream=st.cuda_stream)
+    check(0)
+    hb.open(); hb.consume_columns(cols[1], plain_rows)
+    torch.cuda.synchronize()
+    replay()
+    hb.close(stream=st.cuda_stream)
+    check(0)
+    build(1)
+    for o in (probe, agg, hb):
+        o.destroy()

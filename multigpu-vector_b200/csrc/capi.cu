@@ -34,6 +34,7 @@ mgv_status fail(mgv_status s, const std::string& msg) {
 }
 
 mgv_status cuda_fail(cudaError_t e, const char* what) {
+    (void)cudaGetLastError();  // reported here: the check after the next launch must not find it again
     std::string m = std::string(what) + ": " + cudaGetErrorName(e) + " (" + cudaGetErrorString(e) + ")";
     set_last_error(m);
     if (e == cudaErrorMemoryAllocation) return MGV_ENOMEM;
@@ -569,7 +570,7 @@ mgv_status mgv_op_create_hash_build(mgv_ctx* ctx, const mgv_hash_build_desc* d, 
         if (e == cudaSuccess) e = cudaHostGetDevicePointer(reinterpret_cast<void**>(&o->hb_land_dev), o->hb_land, 0);
         if (e != cudaSuccess) {
             if (o->hb_land) cudaFreeHost(o->hb_land);
-            st = fail(MGV_ENOMEM, "pinned host allocation");
+            st = cuda_fail(e, "pinned host allocation");
         }
     }
     if (st != MGV_OK) {
@@ -627,7 +628,7 @@ mgv_status mgv_op_create_groupby(mgv_ctx* ctx, const mgv_groupby_desc* d, mgv_op
         if (e == cudaSuccess) e = cudaHostGetDevicePointer(reinterpret_cast<void**>(&o->gb_land_dev), o->gb_land, 0);
         if (e != cudaSuccess) {
             if (o->gb_land) cudaFreeHost(o->gb_land);
-            st = fail(MGV_ENOMEM, "pinned host allocation");
+            st = cuda_fail(e, "pinned host allocation");
         }
     }
     if (st != MGV_OK) {
@@ -653,9 +654,10 @@ mgv_status mgv_op_create_partition(mgv_ctx* ctx, const mgv_partition_desc* d, mg
     o->parent = parent;
     mgv_status st = dev_alloc(o, (void**)&o->pt_dev, sizeof(unsigned long long) << d->radix_bits);
     if (st == MGV_OK) st = dev_alloc(o, (void**)&o->pt_acc, sizeof(unsigned long long) * ((1ull << d->radix_bits) + 1));
-    if (st == MGV_OK &&
-        cudaMallocHost(&o->h_res, sizeof(unsigned long long) * ((1ull << d->radix_bits) + 2)) != cudaSuccess)
-        st = fail(MGV_ENOMEM, "pinned host allocation");
+    if (st == MGV_OK) {
+        const cudaError_t e = cudaMallocHost(&o->h_res, sizeof(unsigned long long) * ((1ull << d->radix_bits) + 2));
+        if (e != cudaSuccess) st = cuda_fail(e, "pinned host allocation");
+    }
     if (st != MGV_OK) {
         for (void* p : o->allocs) cudaFree(p);
         delete o;
@@ -688,7 +690,7 @@ mgv_status mgv_op_create_sink(mgv_ctx* ctx, const mgv_sink_desc* d, mgv_op** out
         if (e == cudaSuccess) e = cudaHostGetDevicePointer(reinterpret_cast<void**>(&o->sk_land_dev), o->sk_land, 0);
         if (e != cudaSuccess) {
             if (o->sk_land) cudaFreeHost(o->sk_land);
-            st = fail(MGV_ENOMEM, "pinned host allocation");
+            st = cuda_fail(e, "pinned host allocation");
         }
     }
     if (st != MGV_OK) {

@@ -1189,8 +1189,8 @@ static mgv_status consume_cols(Op* head, const int32_t* const* cols, uint32_t nc
             const int32_t* filt = sel ? cols[sel->sel.col] : nullptr;
             const int32_t bound = sel ? sel->sel.bound : 0;
             const TableView& t = term->table;
-            const bool fresh = term->hb_fresh;
-            term->hb_fresh = false;
+            const bool fresh = term->hb_fresh;  // until the rows of a consume are on their way: one that fails
+                                                // before leaves the clearing to the next consume or the close
             term->hb_landed = false;
             const bool captured = note_capture(term, s);
             RegionJob job{t, cols[kc], pays, filt, bound, 0, 1, kRegionShift, 0, 0, 0};
@@ -1198,6 +1198,7 @@ static mgv_status consume_cols(Op* head, const int32_t* const* cols, uint32_t nc
             // microseconds, less than a second launch costs
             if (fresh && t.nbuckets <= kRegionBuckets && n <= kSmallBuildRows) {
                 MGV_CUDA_TRY(launch_build_small(job, (uint32_t)n, term->hb_land_dev, s, ctx));
+                term->hb_fresh = false;
                 term->hb_landed = true;
                 return MGV_OK;
             }
@@ -1205,6 +1206,7 @@ static mgv_status consume_cols(Op* head, const int32_t* const* cols, uint32_t nc
                 if (fresh) MGV_CUDA_TRY(cudaMemsetAsync(t.meta, 0, 4 * sizeof(unsigned long long), s));
                 if (fresh) MGV_CUDA_TRY(launch_fill_u64(t.slots, 4ull * t.nbuckets, kEmptySlot, s, ctx));
                 MGV_CUDA_TRY(launch_build(cols[kc], pays, filt, bound, sel != nullptr, n, t, s, ctx));
+                term->hb_fresh = false;
                 return MGV_OK;
             }
             // the hash spreads an unpartitioned table's rows evenly: fixed staging shares,
@@ -1254,6 +1256,7 @@ static mgv_status consume_cols(Op* head, const int32_t* const* cols, uint32_t nc
                 MGV_CUDA_TRY(launch_build_regions(nullptr, job, 1, nullptr, 0, n, job.nregions, job.nregions, sc, exact,
                                                   fresh, term->hb_land_dev, zeroed, s, ctx));
             if (!captured) term->rb_zeroed = job.nregions;
+            term->hb_fresh = false;
             term->hb_landed = true;
             return MGV_OK;
         }

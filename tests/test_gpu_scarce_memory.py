@@ -30,3 +30,34 @@ def test_call_after_a_failed_allocation(ctx, torch_cuda, n):
     assert agg.result() == po.Chain(keys, pays).probe_agg(keys, pays)
     for o in (probe, agg, hb):
         o.destroy()
+
+
+@pytest.mark.parametrize("then", ["smaller", "same", "nothing"])
+def test_build_after_a_failed_consume(ctx, torch_cuda, then):
+    """A first consume without room for its scratch leaves the table to be cleared by the next one, or by the close:
+    neither an earlier build's rows nor its counters come back."""
+    torch, n = torch_cuda, 1 << 22
+    old_k, old_p = po.gen_perm(100_000, 0x5EED1202), po.gen_uniform(100_000, 0x5EED1202, 1, 0, 1 << 20)
+    k, p = po.gen_perm(n, 0x5EED1203), po.gen_uniform(n, 0x5EED1203, 1, 0, 1 << 20)
+    pk, pp = po.gen_uniform(50021, 0x5EED1204, 0, 0, 200_000), po.gen_uniform(50021, 0x5EED1204, 1, 0, 1 << 20)
+    cols, probe_cols, old = [[dev(torch, c) for c in side] for side in ((k, p), (pk, pp), (old_k, old_p))]
+    hb = mgv.Op.hash_build(ctx, 0, 1, n)
+    agg = mgv.Op.aggregate(ctx, 1, 2)
+    probe = mgv.Op.hash_probe(ctx, 0, hb, agg)
+    hb.open(); hb.consume_columns(old, len(old_k)); hb.close()
+    hog = leave_free(torch, 16 << 20)
+    hb.open()
+    with pytest.raises(mgv.MgvError) as e:
+        hb.consume_columns(cols, n)
+    assert e.value.status == mgv.ENOMEM
+    del hog
+    torch.cuda.empty_cache()
+    rows = {"smaller": 1000, "same": n, "nothing": 0}[then]
+    if rows:
+        hb.consume_columns(cols, rows)
+    hb.close()
+    assert hb.result().rows == rows
+    probe.open(); probe.consume_columns(probe_cols, len(pk)); probe.close()
+    assert agg.result() == po.Chain(k[:rows], p[:rows]).probe_agg(pk, pp)
+    for o in (probe, agg, hb):
+        o.destroy()

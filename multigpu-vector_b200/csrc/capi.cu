@@ -882,8 +882,9 @@ mgv_status mgv_op_close(mgv_op* o, void* stream) {
             // of a table that a graph holds, the last writer may be a replay that lands nothing
             if (!o->hb_landed || o->graphed) MGV_CUDA_TRY(launch_table_land(o->table, o->hb_land_dev, s, o->ctx));
             MGV_CUDA_TRY(cudaStreamSynchronize(s));
-            const uint32_t w[2] = {o->hb_land->err[0], o->hb_land->err[1]};
-            st = report_device_error(o->ctx, w, s);
+            // the word was read when the counters were, which may be some time ago: an
+            // error may have been reported and cleared since (mgv_ctx_sync)
+            if (o->hb_land->err[0]) st = check_device(o->ctx, s);
             if (st == MGV_OK) hash_build_info(o, o->hb_land->meta);
             return st;
         }

@@ -49,6 +49,7 @@ struct mgv_batch {
     RegionScratch rsc{};
     uint32_t total_regions = 0, max_job_regions = 0;
     uint32_t key_only = 0;  // every query's build side has no payloads: 8-key buckets
+    bool exact = false;     // staging in exact ranges: no room for shares
     BatchOut* d_outs = nullptr;
     BatchItem* d_build_items = nullptr;
     BatchItem* d_probe_items = nullptr;
@@ -116,7 +117,7 @@ mgv_status enqueue_run(mgv_batch* b, cudaStream_t s) {
     layout.t.key_only = b->key_only;
     layout.shift = kRegionShift;
     MGV_CUDA_TRY(launch_build_regions(b->d_jobs, layout, (uint32_t)b->q.size(), b->d_build_items, b->n_build, 0,
-                                      b->total_regions, b->max_job_regions, b->rsc, false, true, nullptr, false, s,
+                                      b->total_regions, b->max_job_regions, b->rsc, b->exact, true, nullptr, false, s,
                                       ctx));
     MGV_CUDA_TRY(launch_batch(b->d_qs, b->d_probe_items, b->n_probe, (int)b->cfg.probe_ctas_per_sm, b->cfg.item_order,
                               s, ctx));
@@ -144,7 +145,7 @@ void sort_rows(std::vector<mgv_group_row>& v) { sort_group_rows(v); }
 constexpr uint32_t kDeviceOrderGroups = kDeviceOrderCap / 2;
 
 mgv_status create_batch(mgv_ctx* ctx, const mgv_query_desc* qs, uint32_t nq, const mgv_batch_config* config,
-                        bool device_order, mgv_batch** out) {
+                        bool exact, bool device_order, mgv_batch** out) {
     if (!ctx || (!qs && nq) || !out) return fail(MGV_EINVAL, "NULL argument");
     *out = nullptr;
     mgv_batch_config cfg{};
@@ -170,6 +171,7 @@ mgv_status create_batch(mgv_ctx* ctx, const mgv_query_desc* qs, uint32_t nq, con
     b->ctx = ctx;
     b->q.assign(qs, qs + nq);
     b->cfg = cfg;
+    b->exact = exact;
 
     // ---- plan the arena ----
     std::vector<uint32_t> nbk(nq), gcap(nq);
@@ -238,7 +240,8 @@ mgv_status create_batch(mgv_ctx* ctx, const mgv_query_desc* qs, uint32_t nq, con
         delete b;
         return fail(MGV_EUNSUPPORTED, "a batch holds fewer than 2^31 build rows");
     }
-    const size_t rsc_off = take(region_scratch_bytes(total_regions, staged, build_total, false, b->key_only != 0));
+    if (exact) staged = build_total;
+    const size_t rsc_off = take(region_scratch_bytes(total_regions, staged, build_total, false, b->key_only != 0, exact));
     const size_t outs_off = take(sizeof(BatchOut) * std::max(nq, 1u));
     b->ordered.assign(nq, 0);
     std::vector<uint32_t> sorts;
@@ -295,7 +298,7 @@ mgv_status create_batch(mgv_ctx* ctx, const mgv_query_desc* qs, uint32_t nq, con
     b->out_counts = reinterpret_cast<uint32_t*>(A + counts_off);
     b->d_qs = reinterpret_cast<ChainDev*>(A + qs_off);
     b->d_jobs = reinterpret_cast<RegionJob*>(A + jobs_off);
-    b->rsc = carve_region_scratch(A + rsc_off, total_regions, staged, build_total, false, b->key_only != 0);
+    b->rsc = carve_region_scratch(A + rsc_off, total_regions, staged, build_total, false, b->key_only != 0, exact);
     b->total_regions = total_regions;
     b->max_job_regions = max_job_regions;
     b->d_outs = reinterpret_cast<BatchOut*>(A + outs_off);
@@ -393,11 +396,11 @@ extern "C" {
 
 mgv_status mgv_batch_create(mgv_ctx* ctx, const mgv_query_desc* qs, uint32_t nq, const mgv_batch_config* config,
                             mgv_batch** out) {
-    mgv_status st = create_batch(ctx, qs, nq, config, true, out);
-    if (st == MGV_ENOMEM) {
-        (void)cudaGetLastError();  // the failed allocation's
-        st = create_batch(ctx, qs, nq, config, false, out);
-    }
+    // scratch a build row in shares of twice the expected rows, in exact ranges:
+    // 28 and 16 bytes, key-only 16 and 12; ordering on the device: 44 a group
+    mgv_status st = create_batch(ctx, qs, nq, config, false, true, out);
+    if (st == MGV_ENOMEM) st = create_batch(ctx, qs, nq, config, true, true, out);
+    if (st == MGV_ENOMEM) st = create_batch(ctx, qs, nq, config, true, false, out);
     return st;
 }
 

@@ -1224,7 +1224,7 @@ static mgv_status consume_cols(Op* head, const int32_t* const* cols, uint32_t nc
             job.cap = region_share(n, job.nregions, t, job.shift);
             uint64_t staged = exact ? n : (uint64_t)job.nregions * job.cap;
             // the scratch is kept by the operator and grown on demand
-            size_t need = region_scratch_bytes(job.nregions, staged, n, true, t.key_only != 0);
+            size_t need = region_scratch_bytes(job.nregions, staged, n, true, t.key_only != 0, exact);
             if (term->rb_bytes < need) {
                 if (term->rb_scratch) {
                     MGV_CUDA_TRY(cudaStreamSynchronize(s));
@@ -1239,14 +1239,15 @@ static mgv_status consume_cols(Op* head, const int32_t* const* cols, uint32_t nc
                     (void)cudaGetLastError();
                     term->rb_exact = exact = true;
                     staged = n;
-                    need = region_scratch_bytes(job.nregions, staged, n, true, t.key_only != 0);
+                    need = region_scratch_bytes(job.nregions, staged, n, true, t.key_only != 0, exact);
                     e = cudaMalloc(&term->rb_scratch, need);
                 }
                 if (e != cudaSuccess) term->rb_scratch = nullptr;
                 MGV_CUDA_TRY(e);
                 term->rb_bytes = need;
             }
-            const RegionScratch sc = carve_region_scratch(term->rb_scratch, job.nregions, staged, n, true, t.key_only != 0);
+            const RegionScratch sc =
+                carve_region_scratch(term->rb_scratch, job.nregions, staged, n, true, t.key_only != 0, exact);
             // a capture runs nothing now: it leaves the scratch as it is
             const bool zeroed = !captured && term->rb_zeroed == job.nregions;
             term->rb_zeroed = 0;  // until every launch is made

@@ -391,7 +391,7 @@ struct RegionScratch {
     uint32_t* start;          // [regions + 1] first staging row of each region (exact ranges)
     unsigned long long* staging;  // {key, payload}, region-major
     unsigned long long* ovf;  // [rows] {key, payload} left for the global insert
-    uint32_t* ovf_job;        // [rows] their jobs; nullptr: one job
+    uint32_t* ovf_job;        // [rows] their jobs; nullptr: one job, or the entries hold the jobs too
 };
 // A table's counters (TableView::meta) and the error word, handed to the host.
 struct TableLanding {
@@ -402,9 +402,9 @@ struct TableLanding {
 void sort_group_rows(std::vector<mgv_group_row>& v);
 inline uint32_t table_regions(const TableView& t) { return (t.nbuckets + kRegionBuckets - 1) / kRegionBuckets; }
 size_t region_zero_bytes(uint32_t regions);
-size_t region_scratch_bytes(uint32_t regions, uint64_t staged, uint64_t rows, bool one_job, bool key_only);
+size_t region_scratch_bytes(uint32_t regions, uint64_t staged, uint64_t rows, bool one_job, bool key_only, bool exact);
 RegionScratch carve_region_scratch(void* base, uint32_t regions, uint64_t staged, uint64_t rows, bool one_job,
-                                   bool key_only);
+                                   bool key_only, bool exact);
 // Staging rows of each region when the ranges are fixed shares.
 uint32_t region_share(uint64_t rows, uint32_t nregions, const TableView& t, uint32_t shift);
 cudaError_t region_build_init();  // once per device: the kernels' shared memory limits

@@ -4,6 +4,7 @@ import pytest
 import mgv
 import pyoracle as po
 from gpu_util import dev
+from querymix import make_query_columns, oracle_answer
 
 pytestmark = pytest.mark.gpu
 
@@ -61,3 +62,37 @@ def test_build_after_a_failed_consume(ctx, torch_cuda, then):
     assert agg.result() == po.Chain(k[:rows], p[:rows]).probe_agg(pk, pp)
     for o in (probe, agg, hb):
         o.destroy()
+
+
+@pytest.mark.parametrize("payloads,lf,share", [(True, 0.5, 0.85), (True, 0.95, 0.93), (False, 0.5, 0.93)])
+def test_batch_without_room_for_staging_shares(ctx, torch_cuda, payloads, lf, share):
+    """A batch that fits with exact staging ranges only is created and takes them: a histogram and a scan more a run,
+    rows that leave their regions (the load factor of 0.95, repeated keys) found by their staging row or key."""
+    torch, mix = torch_cuda, []
+    for i, (nb, dup) in enumerate([(1 << 23, False), (1_000_003, True), (3000, False), (0, False)]):
+        npr = 70_001 + 1000 * i
+        cols = make_query_columns(ctx, torch, nb, npr, 1000, 0x5EED1211 + i, dup)
+        mix.append(dict(nb=nb, npr=npr, bound=700, G=1000, cols=cols))
+    descs = [mgv.query_desc(q["cols"][0], q["nb"], *q["cols"][1:], q["npr"], q["bound"], q["G"],
+                            q["cols"][0] if payloads else None) for q in mix]
+
+    def launches(b):
+        l0 = ctx.launches
+        b.run()
+        return ctx.launches - l0
+
+    config = mgv.BatchConfig(lf, 0, 0, 0, 0, 0)
+    torch.cuda.synchronize()
+    free = torch.cuda.mem_get_info()[0]
+    b = mgv.Batch(ctx, descs, config)
+    arena = free - torch.cuda.mem_get_info()[0]
+    want = launches(b)
+    b.destroy()
+    hog = leave_free(torch, int(share * arena))
+    b = mgv.Batch(ctx, descs, config)
+    assert launches(b) == want + 2
+    b.run()
+    del hog
+    for i, q in enumerate(mix):
+        assert b.result(i) == oracle_answer(q), i
+    b.destroy()

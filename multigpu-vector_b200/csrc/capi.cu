@@ -126,7 +126,7 @@ constexpr uint32_t kHostOrderGroups = 64;
 static mgv_status close_groupby(Op* o, cudaStream_t s) {
     Context* ctx = o->ctx;
     const uint32_t cap = o->gtab.cap;
-    const bool sort = !o->gb_unordered && cap <= kDeviceOrderCap && o->gb.max_groups > kHostOrderGroups;
+    const bool sort = !o->gb_unordered && (cap <= kSmallGroupCap || o->gb_pairs) && o->gb.max_groups > kHostOrderGroups;
     const bool direct = !sort && cap + 1 <= o->gb_land_rows;  // packed rows straight into the landing zone
     o->gb_clean = false;
     if (cap <= kSmallGroupCap) {
@@ -494,8 +494,11 @@ static mgv_op* new_op(Context* ctx, OpKind k) {
     return o;
 }
 
+static size_t align_up(size_t x, size_t to) { return (x + to - 1) / to * to; }
+
 static mgv_status dev_alloc(Op* o, void** p, size_t bytes) {
     cudaError_t e = cudaMalloc(p, bytes);
+    if (e != cudaSuccess) *p = nullptr;
     if (e != cudaSuccess) return cuda_fail(e, "device allocation");
     o->allocs.push_back(*p);
     return MGV_OK;
@@ -616,12 +619,18 @@ mgv_status mgv_op_create_groupby(mgv_ctx* ctx, const mgv_groupby_desc* d, mgv_op
     if (st == MGV_OK) st = dev_alloc(o, (void**)&o->gb_dev_count, 3 * sizeof(uint32_t));
     // landing zone: a larger result's further rows are copied after it
     o->gb_land_rows = std::min<uint32_t>(cap + 1, 1u << 16);
-    if (cap > kSmallGroupCap) {
-        if (st == MGV_OK) st = dev_alloc(o, (void**)&o->gb_dev_rows, sizeof(mgv_group_row) * ((size_t)cap + 1));
-        if (st == MGV_OK && cap <= kDeviceOrderCap)
-            st = dev_alloc(o, (void**)&o->gb_pairs, (2 * sizeof(unsigned long long) + sizeof(uint32_t)) * ((size_t)cap + 1));
-        if (st == MGV_OK && cap <= kDeviceOrderCap && cap + 1 > o->gb_land_rows)
-            st = dev_alloc(o, (void**)&o->gb_dev_more, sizeof(mgv_group_row) * ((size_t)cap + 1 - o->gb_land_rows));
+    if (st == MGV_OK && cap > kSmallGroupCap) {
+        st = dev_alloc(o, (void**)&o->gb_dev_rows, sizeof(mgv_group_row) * ((size_t)cap + 1));
+        // sorting space, with the ordered rows past the landing zone after it;
+        // without room for it the rows are ordered on the host
+        if (st == MGV_OK && cap <= kDeviceOrderCap) {
+            const size_t pairs = 2 * sizeof(unsigned long long) * ((size_t)cap + 1);
+            const size_t order = align_up(sizeof(uint32_t) * ((size_t)cap + 1), sizeof(unsigned long long));
+            const size_t more = sizeof(mgv_group_row) * ((size_t)cap + 1 - o->gb_land_rows);
+            if (dev_alloc(o, (void**)&o->gb_pairs, pairs + order + more) == MGV_OK)
+                o->gb_dev_more = reinterpret_cast<mgv_group_row*>(reinterpret_cast<unsigned char*>(o->gb_pairs) +
+                                                                  pairs + order);
+        }
     }
     if (st == MGV_OK) {
         cudaError_t e = cudaMallocHost(&o->gb_land, sizeof(GroupLanding) + sizeof(mgv_group_row) * (size_t)o->gb_land_rows);

@@ -1,4 +1,5 @@
 """Calls that fail for want of device memory, and the calls after them."""
+import numpy as np
 import pytest
 
 import mgv
@@ -93,6 +94,34 @@ def test_batch_without_room_for_staging_shares(ctx, torch_cuda, payloads, lf, sh
     assert launches(b) == want + 2
     b.run()
     del hog
+    torch.cuda.empty_cache()
     for i, q in enumerate(mix):
         assert b.result(i) == oracle_answer(q), i
     b.destroy()
+
+
+@pytest.mark.parametrize("groups", [1 << 18, 1 << 20])
+def test_groupby_without_room_for_sorting(ctx, torch_cuda, groups):
+    """A group-by with room for its table and rows but not for sorting space is created; the host orders its rows."""
+    torch, n = torch_cuda, 3_000_017
+    group = po.gen_uniform(n, 0x5EED1221, 0, -groups // 2, groups)
+    value = po.gen_uniform(n, 0x5EED1221, 1, 0, 1 << 20)
+    cols = [dev(torch, group), dev(torch, value)]
+    torch.cuda.synchronize()
+    free = torch.cuda.mem_get_info()[0]
+    gb = mgv.Op.groupby(ctx, 0, 1, groups)
+    need = free - torch.cuda.mem_get_info()[0]
+    gb.destroy()
+    hog = leave_free(torch, int(0.8 * need))  # table 20 bytes a slot, rows 24; sorting space 20 to 43
+    gb = mgv.Op.groupby(ctx, 0, 1, groups)
+    l0 = ctx.launches
+    gb.open(); gb.close()
+    assert ctx.launches - l0 == 2  # the reset, the packing
+    gb.open(); gb.consume_columns(cols, n); gb.close()
+    del hog
+    torch.cuda.empty_cache()
+    g, inverse, count = np.unique(group, return_inverse=True, return_counts=True)
+    total = np.zeros(len(g), np.int64)
+    np.add.at(total, inverse, value.astype(np.int64))
+    assert gb.result() == list(zip(g.tolist(), total.tolist(), count.tolist()))
+    gb.destroy()

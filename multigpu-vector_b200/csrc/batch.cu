@@ -76,7 +76,7 @@ struct mgv_batch {
     struct PlainQuery {
         mgv_op *hb = nullptr, *gb = nullptr, *probe = nullptr, *sel = nullptr;
         std::vector<mgv_group_row> rows;
-        bool sorted = false;  // by the group-by's close, else when read
+        bool sorted = false;  // by the group-by's close, else in each read
     };
     std::vector<PlainQuery> plain;
 };
@@ -473,7 +473,7 @@ mgv_status mgv_batch_run_plain(mgv_batch* b, void* stream) {
         if (st != MGV_OK) return st;
     }
     b->last_ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
-    // kept as closed (unordered); ordered when read, as the batch's own rows
+    // kept as closed: in group order, or (few groups, very many) ordered in each read
     for (uint32_t i = 0; i < nq; ++i) {
         const Op* g = static_cast<Op*>(b->plain[i].gb);
         b->plain[i].rows.assign(g->gb_view, g->gb_view + g->gb_n);
@@ -487,23 +487,24 @@ mgv_status mgv_batch_result(mgv_batch* b, uint32_t q, int plain, mgv_group_row* 
     if (q >= b->q.size()) return fail(MGV_EINVAL, "no such query");
     const mgv_group_row* v = nullptr;
     uint64_t n = 0;
+    bool in_order = false;
     std::vector<mgv_group_row> sorted;
     if (plain) {
         if (b->plain.empty()) return fail(MGV_ESTATE, "the plain pipeline has not run");
-        auto& p = b->plain[q];
-        if (!p.sorted) sort_rows(p.rows);
-        p.sorted = true;
+        const auto& p = b->plain[q];
         v = p.rows.data();
         n = p.rows.size();
+        in_order = p.sorted;
     } else {
         if (!b->warmed) return fail(MGV_ESTATE, "the batch has not run");
         v = b->h_rows + b->out_offset[q];
         n = std::min<uint32_t>(b->h_counts[q], b->q[q].max_groups);
-        if (!b->ordered[q]) {
-            sorted.assign(v, v + n);
-            sort_rows(sorted);
-            v = sorted.data();
-        }
+        in_order = b->ordered[q] != 0;
+    }
+    if (!in_order) {  // in a copy: several threads may read one query
+        sorted.assign(v, v + n);
+        sort_rows(sorted);
+        v = sorted.data();
     }
     if (rows) *rows = n;
     if (out) std::memcpy(out, v, sizeof(mgv_group_row) * std::min<uint64_t>(cap, n));

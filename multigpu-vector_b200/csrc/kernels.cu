@@ -18,16 +18,14 @@ namespace mgv {
 constexpr int kBlock = 256;
 
 int blocks_per_sm(const void* kernel, int block, size_t smem, const Context* ctx) {
-    std::lock_guard<std::mutex> lk(ctx->fit_mu);
-    for (const Context::Fit& f : ctx->fits)
-        if (f.kernel == kernel && f.block == block && f.smem == smem) return f.per_sm;
+    int per_sm = 0;
+    if (ctx->fits.find(kernel, block, smem, &per_sm)) return per_sm;
     cudaFuncAttributes fa;
     if (cudaFuncGetAttributes(&fa, kernel) == cudaSuccess)
         (void)cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                    (int)(ctx->prop.sharedMemPerBlockOptin - fa.sharedSizeBytes));
-    int per_sm = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, block, smem) != cudaSuccess || per_sm < 1) return 1;
-    ctx->fits.push_back(Context::Fit{kernel, block, smem, per_sm});
+    ctx->fits.add(kernel, block, smem, per_sm);
     return per_sm;
 }
 

@@ -11,6 +11,7 @@
 #include <vector>
 
 #include "../../include/mgv.h"
+#include "launch_fits.h"
 
 namespace mgv {
 
@@ -123,15 +124,7 @@ struct Context {
     mgv_batch_config batch_tuned{};  // the batch autotuner's last choice
     bool has_batch_tuned = false;
     std::mutex mu;
-    // CTAs per SM of each launch shape used so far (blocks_per_sm)
-    struct Fit {
-        const void* kernel;
-        int block;
-        size_t smem;
-        int per_sm;
-    };
-    mutable std::mutex fit_mu;
-    mutable std::vector<Fit> fits;
+    mutable LaunchFits fits;  // CTAs per SM of the launch shapes used lately (blocks_per_sm)
 };
 
 enum class OpKind { Select, Aggregate, HashBuild, HashProbe, Sink, Groupby, Partition };

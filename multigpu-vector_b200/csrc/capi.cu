@@ -724,6 +724,9 @@ mgv_status mgv_op_destroy(mgv_op* o) {
     if (!o) return MGV_OK;
     cudaSetDevice(o->ctx->device);
     cudaStreamSynchronize(o->ctx->stream);
+    // an operator destroyed while open may have work on any stream, and a build's
+    // writes into the pinned memory that goes back below
+    if (o->state == OpState::Open) cudaDeviceSynchronize();
     if (o->kind == OpKind::Sink) {
         sink_finish_drain(o);
         sink_return_buffers(o);

@@ -1239,8 +1239,12 @@ static mgv_status consume_cols(Op* head, const int32_t* const* cols, uint32_t nc
             size_t need = region_scratch_bytes(job.nregions, staged, n, true, t.key_only != 0, exact);
             if (term->rb_bytes < need) {
                 if (term->rb_scratch) {
-                    MGV_CUDA_TRY(cudaStreamSynchronize(s));
-                    MGV_CUDA_TRY(cudaFree(term->rb_scratch));
+                    if (term->graphed) {  // a replay may still come to it: kept until the operator goes
+                        term->allocs.push_back(term->rb_scratch);
+                    } else {
+                        MGV_CUDA_TRY(cudaStreamSynchronize(s));
+                        MGV_CUDA_TRY(cudaFree(term->rb_scratch));
+                    }
                     term->rb_scratch = nullptr;
                     term->rb_bytes = 0;
                 }

@@ -770,6 +770,13 @@ static bool note_capture(Op* o, cudaStream_t s) {
     return c;
 }
 
+// A hash build's table and counters, empty.
+static mgv_status clear_table(Op* o, cudaStream_t s) {
+    MGV_CUDA_TRY(cudaMemsetAsync(o->table.meta, 0, 4 * sizeof(unsigned long long), s));
+    MGV_CUDA_TRY(launch_fill_u64(o->table.slots, 4ull * o->table.nbuckets, kEmptySlot, s, o->ctx));
+    return MGV_OK;
+}
+
 // Resets one operator's device state (at_open).
 static mgv_status op_reset(Op* o, cudaStream_t s) {
     switch (o->kind) {
@@ -787,6 +794,10 @@ static mgv_status op_reset(Op* o, cudaStream_t s) {
             o->hb_fresh = true;
             o->hb_landed = false;
             o->unique = false;
+            // a replay may be all that is built, which the close would not know:
+            // of an operator that a graph holds, the open clears the table itself
+            o->hb_cleared = o->graphed && !capturing(s);
+            if (o->hb_cleared) return clear_table(o, s);
             break;
         case OpKind::Sink: {
             mgv_status st = sink_return_buffers(o);
@@ -870,11 +881,11 @@ mgv_status mgv_op_close(mgv_op* o, void* stream) {
         st = sink_finish_drain(o);
         if (st != MGV_OK) return st;
     }
-    if (o->kind == OpKind::HashBuild && o->hb_fresh) {  // nothing was built: clear the table now
-        MGV_CUDA_TRY(cudaMemsetAsync(o->table.meta, 0, 4 * sizeof(unsigned long long), s));
-        MGV_CUDA_TRY(launch_fill_u64(o->table.slots, 4ull * o->table.nbuckets, kEmptySlot, s, o->ctx));
-        o->hb_fresh = false;
+    if (o->kind == OpKind::HashBuild && o->hb_fresh && !o->hb_cleared) {  // nothing was built: clear the table now
+        st = clear_table(o, s);
+        if (st != MGV_OK) return st;
     }
+    o->hb_fresh = false;
     if (!o->parent) {  // terminal: wait, check the device error word, read results
         if (o->kind == OpKind::Aggregate) {
             // one kernel hands the error word and the sums to the host and leaves
@@ -1216,8 +1227,8 @@ static mgv_status consume_cols(Op* head, const int32_t* const* cols, uint32_t nc
                 return MGV_OK;
             }
             if (n < kRegionBuildMinRows || n >= (1ull << 31) || table_regions(t) > kMaxRegionsPerJob) {
-                if (fresh) MGV_CUDA_TRY(cudaMemsetAsync(t.meta, 0, 4 * sizeof(unsigned long long), s));
-                if (fresh) MGV_CUDA_TRY(launch_fill_u64(t.slots, 4ull * t.nbuckets, kEmptySlot, s, ctx));
+                const mgv_status st = fresh ? clear_table(term, s) : MGV_OK;
+                if (st != MGV_OK) return st;
                 MGV_CUDA_TRY(launch_build(cols[kc], pays, filt, bound, sel != nullptr, n, t, s, ctx));
                 term->hb_fresh = false;
                 return MGV_OK;

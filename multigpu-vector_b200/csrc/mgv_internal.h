@@ -196,6 +196,7 @@ struct Op {
     unsigned long long* pt_acc = nullptr; // [1 + P] rows stored, rows per partition
     std::vector<uint64_t> pt_hist;        // rows per partition (read back at close)
     bool hb_fresh = false;  // opened, nothing consumed yet: the table and its counters are not cleared yet
+    bool hb_cleared = false;  // the open cleared them (a graph holds the operator)
     bool hb_landed = false;  // the last consume's kernels hand the table's counters to the host
     struct TableLanding* hb_land = nullptr;  // pinned, mapped
     struct TableLanding* hb_land_dev = nullptr;

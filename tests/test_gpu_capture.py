@@ -127,3 +127,43 @@ def test_replayed_build_is_closed_by_its_own_counters(ctx, torch_cuda, captured_
     build(1)
     for o in (probe, agg, hb):
         o.destroy()
+
+
+@pytest.mark.parametrize("rows", [1000, 30_000, 150_001])
+def test_build_by_a_replay_alone(ctx, torch_cuda, rows):
+    """Open, replay of a captured build, close: the table holds the replay's rows.  Open, close: it is empty."""
+    torch, room = torch_cuda, 150_001
+    side = po.gen_perm(rows, 0x5EED1121), po.gen_uniform(rows, 0x5EED1121, 1, 0, 1 << 20)
+    other = po.gen_perm(room, 0x5EED1122), po.gen_uniform(room, 0x5EED1122, 1, 0, 1 << 20)
+    pk, pp = po.gen_uniform(20011, 0x5EED1123, 0, 0, 1 << 17), po.gen_uniform(20011, 0x5EED1123, 1, 0, 1 << 20)
+    cols, other_cols, probe_cols = [[dev(torch, c) for c in s] for s in (side, other, (pk, pp))]
+    none = [c[:0] for c in side]
+    hb = mgv.Op.hash_build(ctx, 0, 1, room)
+    agg = mgv.Op.aggregate(ctx, 1, 2)
+    probe = mgv.Op.hash_probe(ctx, 0, hb, agg)
+
+    def check(s):
+        assert hb.result().rows == len(s[0])
+        probe.open(); probe.consume_columns(probe_cols, len(pk)); probe.close()
+        assert agg.result() == po.Chain(*s).probe_agg(pk, pp)
+
+    def build(s, c):
+        hb.open(); hb.consume_columns(c, len(s[0])); hb.close()
+        check(s)
+
+    build(side, cols)
+    build(other, other_cols)
+    st, replay = capture(torch, hb, cols, rows)
+    replay()
+    hb.close(stream=st.cuda_stream)
+    check(side)
+    for _ in range(2):
+        build(other, other_cols)
+        hb.open(stream=st.cuda_stream)
+        replay()
+        hb.close(stream=st.cuda_stream)
+        check(side)
+        hb.open(); hb.close()
+        check(none)
+    for o in (probe, agg, hb):
+        o.destroy()

@@ -265,19 +265,16 @@ __global__ void __launch_bounds__(kRBlock) k_region_scatter(const RegionJob* __r
 // ---- sorted tiles -------------------------------------------------------------
 
 constexpr int kTileBlock = 512;
-// Rows per thread, held in registers from load to placement.
-template <bool KO>
-constexpr int tile_rows() { return 16; }
-template <bool KO>
-constexpr uint32_t tile_size() { return kTileBlock * tile_rows<KO>(); }
+constexpr int kTileRows = 16;  // per thread, held in registers from load to placement
+constexpr uint32_t kTileSize = kTileBlock * kTileRows;
 constexpr uint32_t kTileRegions = 4096;   // most regions a tile sorts: runs of two rows on average
 constexpr uint32_t kTileCounters = 1024;  // rank counters are replicated per lane while they are at most this many
 
 // A tile's sorting space: two CTAs fit per SM up to 1024 regions.
 template <bool KO>
 struct TileSpace {
-    typename std::conditional<KO, uint32_t, unsigned long long>::type* val;  // [tile_size] rows in region order
-    uint16_t* reg;     // [tile_size] region of each sorted position
+    typename std::conditional<KO, uint32_t, unsigned long long>::type* val;  // [kTileSize] rows in region order
+    uint16_t* reg;     // [kTileSize] region of each sorted position
     uint32_t* off;     // [regions * copies] counts, then first sorted positions
     uint32_t* base;    // [regions] region row of sorted position 0 (mod 2^32)
     uint32_t copies;   // rank counters per region: lane & (copies - 1) picks one
@@ -302,15 +299,15 @@ constexpr bool tile_counters_fit() {
 static_assert(tile_counters_fit(), "a job's counters fit the space of every launch it can be part of");
 template <bool KO>
 __host__ __device__ constexpr size_t tile_smem(uint32_t regions) {
-    return (KO ? 6ull : 10ull) * tile_size<KO>() + tile_counter_bytes(regions) + 4ull * regions;
+    return (KO ? 6ull : 10ull) * kTileSize + tile_counter_bytes(regions) + 4ull * regions;
 }
 template <bool KO>
 __device__ __forceinline__ TileSpace<KO> tile_space(unsigned char* base, uint32_t regions) {
     TileSpace<KO> s;
     s.val = reinterpret_cast<decltype(s.val)>(base);
-    s.reg = reinterpret_cast<uint16_t*>(s.val + tile_size<KO>());
+    s.reg = reinterpret_cast<uint16_t*>(s.val + kTileSize);
     s.copies = tile_copies(regions);
-    s.off = reinterpret_cast<uint32_t*>(s.reg + tile_size<KO>());
+    s.off = reinterpret_cast<uint32_t*>(s.reg + kTileSize);
     s.base = s.off + regions * s.copies;
     return s;
 }
@@ -324,7 +321,7 @@ __device__ __forceinline__ void side_list_row(const TableView& t, int32_t pay, u
     else set_error(err, kDevTableFull, 1);
 }
 
-// Rows [lo, hi) (at most tile_size) of a job to their regions: ranks by shared
+// Rows [lo, hi) (at most kTileSize) of a job to their regions: ranks by shared
 // atomics, positions by a scan, one reserve(region, rows) -> first row per
 // region, then put(region, row, value) in region order, so that a warp's
 // stores are runs.  Every thread of the CTA calls it.
@@ -339,10 +336,10 @@ __device__ __forceinline__ void sort_tile(const RegionJob& job, const TileSpace<
     const int32_t* const pays = !KO && job.pays ? job.pays + lo : nullptr;
     const int32_t* const filt = job.filt ? job.filt + lo : nullptr;
     const int32_t bound = job.bound;
-    int32_t key[tile_rows<KO>()], pay[tile_rows<KO>()];
-    uint32_t at[tile_rows<KO>()];  // region << 16 | rank, ~0 for no row
+    int32_t key[kTileRows], pay[kTileRows];
+    uint32_t at[kTileRows];  // region << 16 | rank, ~0 for no row
 #pragma unroll
-    for (int u = 0; u < tile_rows<KO>(); ++u) {
+    for (int u = 0; u < kTileRows; ++u) {
         const uint32_t i = u * kTileBlock + threadIdx.x;
         key[u] = i < n ? __ldg(keys + i) : kEmptyKey;
         pay[u] = pays && i < n ? __ldg(pays + i) : 0;
@@ -352,12 +349,12 @@ __device__ __forceinline__ void sort_tile(const RegionJob& job, const TileSpace<
     const uint32_t copy = lane_id() & (ts.copies - 1);
     bool reserved = false;
 #pragma unroll
-    for (int u = 0; u < tile_rows<KO>(); ++u) {
+    for (int u = 0; u < kTileRows; ++u) {
         reserved |= key[u] == kEmptyKey && u * kTileBlock + threadIdx.x < n;
         at[u] = at[u] == 0 && key[u] != kEmptyKey ? region(key[u]) << 16 : ~0u;
     }
 #pragma unroll
-    for (int u = 0; u < tile_rows<KO>(); ++u)
+    for (int u = 0; u < kTileRows; ++u)
         if (at[u] != ~0u) at[u] |= atomicAdd(ts.off + (at[u] >> 16) * ts.copies + copy, 1u);
     if (reserved) {  // rare: the rows are read again, so that the common path holds nothing for them
 #pragma unroll 1
@@ -375,7 +372,7 @@ __device__ __forceinline__ void sort_tile(const RegionJob& job, const TileSpace<
         ts.base[r] = (c ? reserve(r, c) : 0u) - first;
     }
 #pragma unroll
-    for (int u = 0; u < tile_rows<KO>(); ++u) {
+    for (int u = 0; u < kTileRows; ++u) {
         if (at[u] == ~0u) continue;
         const uint32_t r = at[u] >> 16, p = ts.off[r * ts.copies + copy] + (at[u] & 0xffffu);
         if constexpr (KO) ts.val[p] = (uint32_t)key[u];
@@ -409,8 +406,8 @@ __global__ void __launch_bounds__(kTileBlock, 2)
         const HomeFn home(sj);
         const StageFn<KO> stage(out, sj, item.q);
         uint32_t* const cursor = out.cursor + sj.region0;
-        for (uint64_t lo = item.lo; lo < item.hi; lo += tile_size<KO>())
-            sort_tile<KO>(sj, ts, sj.nregions, lo, min(item.hi, lo + tile_size<KO>()), err, nullptr,
+        for (uint64_t lo = item.lo; lo < item.hi; lo += kTileSize)
+            sort_tile<KO>(sj, ts, sj.nregions, lo, min(item.hi, lo + kTileSize), err, nullptr,
                           [&](int32_t key) { return home.region(key); },
                           [&](uint32_t r, uint32_t c) { return atomicAdd(cursor + r, c); }, stage);
     }
@@ -872,15 +869,15 @@ __global__ void __launch_bounds__(kTileBlock, 2) k_region_part_scatter(const __g
         if (threadIdx.x == 0) side_rows = 0;
         __syncthreads();
         // 1. rows per region
-        for (uint64_t i0 = lo + threadIdx.x; i0 < hi; i0 += tile_size<KO>()) {
-            int32_t key[tile_rows<KO>()];
+        for (uint64_t i0 = lo + threadIdx.x; i0 < hi; i0 += kTileSize) {
+            int32_t key[kTileRows];
 #pragma unroll
-            for (int u = 0; u < tile_rows<KO>(); ++u) {
+            for (int u = 0; u < kTileRows; ++u) {
                 const uint64_t i = i0 + (uint64_t)u * kTileBlock;
                 key[u] = i < hi ? __ldg(job.keys + i) : kEmptyKey;
             }
 #pragma unroll
-            for (int u = 0; u < tile_rows<KO>(); ++u)
+            for (int u = 0; u < kTileRows; ++u)
                 if (key[u] != kEmptyKey) atomicAdd(ts.off + region(key[u]) * ts.copies + copy, 1u);
         }
         __syncthreads();
@@ -892,8 +889,8 @@ __global__ void __launch_bounds__(kTileBlock, 2) k_region_part_scatter(const __g
         }
         if (p == P - 1 && threadIdx.x == 0) start[(uint64_t)P * rpp] = (uint32_t)hi;
         // 2. the rows, region-major
-        for (uint64_t t0 = lo; t0 < hi; t0 += tile_size<KO>())
-            sort_tile<KO>(job, ts, rpp, t0, min(hi, t0 + tile_size<KO>()), err, &side_rows, region,
+        for (uint64_t t0 = lo; t0 < hi; t0 += kTileSize)
+            sort_tile<KO>(job, ts, rpp, t0, min(hi, t0 + kTileSize), err, &side_rows, region,
                           [&](uint32_t r, uint32_t c) {  // one thread per region: no atomic
                               const uint32_t at = cur[r];
                               cur[r] = at + c;
@@ -1051,11 +1048,10 @@ cudaError_t launch_build_regions(const RegionJob* d_jobs, const RegionJob& table
     const void* k = tiles ? (ko ? (const void*)k_region_tile_scatter<true> : (const void*)k_region_tile_scatter<false>)
                           : (ko ? (const void*)k_region_scatter<true> : (const void*)k_region_scatter<false>);
     const uint64_t ctas = (uint64_t)occupancy_grid(k, tiles ? kTileBlock : kRBlock, smem, ctx);
-    const uint64_t tile = ko ? tile_size<true>() : tile_size<false>();
     uint64_t rpi = 0;
     if (!items && n) {
         // whole tiles dealt evenly over the CTAs, or items worth zeroing and flushing their region counters
-        if (tiles) rpi = (n - 1) / (ctas * ((n - 1) / (ctas * tile) + 1)) + 1;
+        if (tiles) rpi = (n - 1) / (ctas * ((n - 1) / (ctas * kTileSize) + 1)) + 1;
         else rpi = std::max<uint64_t>({8ull * max_job_regions, 4096, n / (2ull * ctx->prop.multiProcessorCount) + 1});
         nitems = (uint32_t)((n + rpi - 1) / rpi);
     }

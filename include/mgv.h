@@ -97,7 +97,7 @@ typedef struct mgv_tuning {
                                        per SM, 1..8 (0 = the default, 2)             */
     uint32_t select_compact;        /* select -> aggregate: 0 = masked fold of every row
                                        (the default), 1 = warp-ballot compaction of the
-                                       qualifying rows into 128-row vectors that the
+                                       qualifying rows into 64-row vectors that the
                                        aggregate reads (unstable_select::consume_warp,
                                        src/operators/select3.cu:19-85); same results */
 } mgv_tuning;

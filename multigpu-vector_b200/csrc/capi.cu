@@ -118,8 +118,9 @@ void sort_group_rows(std::vector<mgv_group_row>& v) {
 // the next open has nothing to clear.  A table of up to kSmallGroupCap slots
 // takes one kernel of one CTA (a table that size is read in a few
 // microseconds); a larger one is packed by the whole GPU, ordered by one CTA
-// and written out by many; one past kDeviceOrderCap slots (half a GiB of sorting space and up) is
-// ordered by the host when its result is read, and so is one of at most
+// and written out by many; one past kDeviceOrderCap slots (84 MB of sorting
+// space and up, and 99 for ordered rows) is ordered by the host when its result
+// is read, and so are one that had no room for that space and one of at most
 // kHostOrderGroups groups (a microsecond on the host).
 constexpr uint32_t kHostOrderGroups = 64;
 
@@ -922,7 +923,7 @@ mgv_status mgv_op_close(mgv_op* o, void* stream) {
     if (o->kind == OpKind::Partition) {
         // the device's totals (and any overflow of max_rows), then the stored
         // rows -- every consume's run partition-major -- go to the parent chain;
-        // a hash build on the same radix bits scatters them by sorted warp tiles
+        // a hash build on the same radix bits stages a single run partition by partition
         o->pt_close_stream = s;
         if (!o->pt_filtered && o->pt_offered <= o->pt.max_rows) {
             // every consumed row was stored: the replay needs nothing from the device, so
@@ -1262,7 +1263,8 @@ static mgv_status consume_cols(Op* head, const int32_t* const* cols, uint32_t nc
                 term->rb_zeroed = 0;
                 cudaError_t e = cudaMalloc(&term->rb_scratch, need);
                 if (e == cudaErrorMemoryAllocation && !exact) {
-                    // the shares take up to 24 bytes a row, exact ranges 16 (key-only: 16, 12)
+                    // shares take up to 24 bytes a row and 256 rows a region, exact ranges
+                    // 16 bytes a row (key-only: 16 and 12)
                     (void)cudaGetLastError();
                     term->rb_exact = exact = true;
                     staged = n;

@@ -735,8 +735,9 @@ constexpr size_t chain_ring_bytes() {
     return SEL ? (size_t)(chain_block<TERM>() / 32) * kIdRing * sizeof(uint32_t) : 0;
 }
 
-// UNIQUE: the table is known to have no duplicate keys (a sink's probe has no
-// flush, a call, inside its rounds then).
+// UNIQUE: the table is known to have no duplicate keys: a row has one match at
+// most, so the room made before a vector is enough and the rounds of a sink's
+// probe hold no flush.
 template <bool SEL, bool PROBE, int TERM, bool UNIQUE = false>
 __global__ void __launch_bounds__(chain_block<TERM>(), TERM == kTermSink ? 2 : 1)
     k_chain(const __grid_constant__ ChainDev a, uint32_t* err) {

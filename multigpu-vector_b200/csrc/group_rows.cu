@@ -2,14 +2,16 @@
 // ordered by group on the device and written straight into pinned, mapped
 // host memory, with the table left empty for the next open.
 //
-// Ordering is a sort of {group, source} pairs by one CTA per result: a result
-// has at most a few tens of thousands of groups, so a device-wide sort would
-// be launches and waits, and results of a batch run side by side on different
-// SMs.  On the host it cost about 35 us per 4096 groups and was half of a
-// batch's time with its results read (366 K groups of 64 queries: 3.1 ms; here
-// 64 us for the largest of them, 60 K groups).  The ordered rows are written
-// to the host by many CTAs, at the host link's rate (8.8 MB in 118 us): one
-// SM's stores to host memory reach about 8 GB/s.
+// Ordering is a sort of {group, source} pairs by one CTA per result: most
+// results have at most a few tens of thousands of groups, so a device-wide sort
+// would be launches and waits, and results of a batch run side by side on
+// different SMs.  (Of a million groups one CTA still takes a third of the time
+// that the host does: kDeviceOrderCap.)  On the host it cost about 35 us per
+// 4096 groups and was half of a batch's time with its results read (366 K
+// groups of 64 queries: 3.1 ms; here 64 us for the largest of them, 60 K
+// groups).  The ordered rows are written to the host by many CTAs, at the host
+// link's rate (8.8 MB in 118 us): one SM's stores to host memory reach about
+// 8 GB/s.
 #include <cuda_runtime.h>
 
 #include <algorithm>

@@ -452,7 +452,13 @@ struct GroupSortJob {
     uint32_t out_rows;
 };
 constexpr uint32_t kSmallGroupCap = 2048;      // slots of a table that one CTA closes
-constexpr uint32_t kDeviceOrderCap = 1u << 21;  // slots of the largest table ordered on the device
+// Slots of the largest table ordered on the device, by one CTA.  Close and read
+// of a result on the host / on the device, us, dense and sparse group ids: 2^13
+// groups 117 / 51 and 140 / 89, 2^16 1218 / 260 and 1530 / 538, 2^18 5742 / 2579
+// and 7060 / 3000, 2^20 34085 / 10816 and 35070 / 11930.  (The close alone is the
+// longer one of the two from 2^17 groups on: 505 / 670; 3699 / 8594 for 2^20.)
+// Past this the sorting space is what counts against it.
+constexpr uint32_t kDeviceOrderCap = 1u << 21;
 cudaError_t group_rows_init();  // once per device: the kernels' shared memory limits
 cudaError_t launch_group_reset(const GroupTableView& gt, uint32_t* count, cudaStream_t s, Context* ctx);
 cudaError_t launch_group_close(const GroupTableView& gt, GroupLanding* land, bool sort, cudaStream_t s, Context* ctx);

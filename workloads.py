@@ -126,7 +126,7 @@ def run_select(args, mgv, torch, ctx, bench, clk, emit=True):
     launches = (ctx.launches - launches0) * args.steps // (args.warmup + args.steps)
     cnt, s = agg.result()
     # the same select through the warp-ballot compaction (qualifying rows packed
-    # into 128-row vectors that the aggregate reads): untimed for the headline
+    # into 64-row vectors that the aggregate reads): untimed for the headline
     tuning0 = ctx.tuning()
     ctx.set_tuning(select_compact=1)
     try:
@@ -172,7 +172,7 @@ def run_select(args, mgv, torch, ctx, bench, clk, emit=True):
     extra = {"roofline": {"bound": "hbm", "achieved": 8 * n / kt / 1e9, "peak": peak, "unit": "GB/s",
                           "frac": 8 * n / kt / 1e9 / peak, "peak_kind": kind, "kernel_ms": 1000 * kt,
                           "algorithmic_bytes_per_launch": 8 * n, "kernel": "k_select_agg"},
-             "ballot_path": {"kernel": "k_chain<select, aggregate> (warp-ballot compaction into 128-row vectors; "
+             "ballot_path": {"kernel": "k_chain<select, aggregate> (warp-ballot compaction into 64-row vectors; "
                                        "mgv_tuning.select_compact = 1)", "kernel_ms": 1000 * bkt,
                              "achieved_gbs": 8 * n / bkt / 1e9, "frac": 8 * n / bkt / 1e9 / peak,
                              "checked": "COUNT and SUM equal the masked fold's (and so the oracle's)"},

@@ -606,7 +606,8 @@ __device__ __forceinline__ void chain_windows(const ChainDev& a, bool unique, ui
                 if (live[j]) ld_bucket(slots + 4ull * b[j], w[j]);
             }
             const bool ko = a.table.key_only != 0;  // eight keys per bucket, payloads 0
-            for (uint32_t round = 0; round <= nbuckets; ++round) {
+            // (at most the whole table: without a free slot in it no run ends by itself)
+            for (uint32_t round = 0; round < nbuckets; ++round) {
 #pragma unroll
                 for (int j = 0; j < kVecRows; ++j) {
                     const uint32_t k = (uint32_t)key[j];
